@@ -94,34 +94,83 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 
-// Thread mapping: 16 warps; a half-warp (16 lanes x 8 columns) covers one 128-wide weight row.
-// In the two hidden layers warp w owns output rows [8w, 8w+8): load j of a lane belongs to
-// row 8w + 2j + (lane >> 4). In the last layer warp w owns rows 2w and 2w+1.
-constexpr int kMlpWarps = kHashDecodeThreads / 32;   // 16
-constexpr int kRowLoads = kHidden / kMlpWarps / 2;   // 4 loads per lane and hidden layer
+// Sums of N rows (N = 1, 2, 4 or 8) over the 16 lanes of a half-warp: at every step of the butterfly a lane hands half of
+// its rows to its partner and keeps the other half, so N rows take N - 1 + log2(16 / N) shuffles instead of 4 N and every
+// lane ends up with the sum of one row, row spread_row<N>(sub). Each row is added up in the order of half_warp_sum.
+template <int N>
+__device__ __forceinline__ float spread_sum(const float (&s)[N], int sub) {
+    if constexpr (N == 1) {
+        return half_warp_sum(s[0]);
+    } else {
+        float r[N / 2];
+        const bool upper = (sub & 8) != 0;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float send = upper ? s[i] : s[i + N / 2], keep = upper ? s[i + N / 2] : s[i];
+            r[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        }
+        if constexpr (N == 2) {
+            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 4);
+            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 2);
+            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 1);
+            return r[0];
+        } else {
+            float t[N / 4];
+            const bool upper4 = (sub & 4) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 4; ++i) {
+                const float send = upper4 ? r[i] : r[i + N / 4], keep = upper4 ? r[i + N / 4] : r[i];
+                t[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            }
+            if constexpr (N == 4) {
+                t[0] += __shfl_xor_sync(0xffffffffu, t[0], 2);
+            } else {
+                static_assert(N == 8, "up to 8 rows");
+                const bool upper2 = (sub & 2) != 0;
+                const float send = upper2 ? t[0] : t[1], keep = upper2 ? t[1] : t[0];
+                t[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+            }
+            return t[0] + __shfl_xor_sync(0xffffffffu, t[0], 1);
+        }
+    }
+}
+// the row whose sum lane `sub` of a half-warp ends up with; 16 / N lanes hold the same one, the first of them has
+// sub % (16 / N) == 0
+template <int N>
+__device__ __forceinline__ int spread_row(int sub) { return sub / (16 / N); }
 
-// One head's MLP held in the registers of a 512-thread CTA.
-template <typename WT>
+// Thread mapping: kWarps warps; a half-warp (16 lanes x 8 columns) covers one 128-wide weight row.
+// In the two hidden layers a warp owns 128 / kWarps consecutive output rows: load j of a lane belongs to
+// row 2j + (lane >> 4) of them. In the last layer it owns 32 / kWarps rows in the same way.
+constexpr int kMlpWarps = kHashDecodeThreads / 32;   // 16
+template <int kWarps>
+struct MlpRows {
+    static constexpr int kHid = kHidden / kWarps / 2;   // rows per half-warp in a hidden layer
+    static constexpr int kOut = kCodeBits / kWarps / 2;  // ... in the last one
+};
+
+// One head's MLP held in the registers of a CTA of kWarps warps.
+template <typename WT, int kWarps = kMlpWarps>
 struct MlpRegs {
-    Row8<WT> w0[kRowLoads], w1[kRowLoads], w2;
-    float b0[kRowLoads], b1[kRowLoads], b2;
+    static constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
+    Row8<WT> w0[kHid], w1[kHid], w2[kOut];
+    float b0, b1, b2;  // biases of the rows whose sums this lane ends up with
 
     // All three layers are fetched back to back so that their DRAM latency is paid once.
-    __device__ __forceinline__ void load(const WT* W, const float* bias, int warp, int half, int col) {
+    __device__ __forceinline__ void load(const WT* W, const float* bias, int warp, int lane) {
+        const int half = lane >> 4, sub = lane & 15, col = sub * 8;
 #pragma unroll
-        for (int j = 0; j < kRowLoads; ++j) {
-            const int row = warp * (2 * kRowLoads) + 2 * j + half;
+        for (int j = 0; j < kHid; ++j) {
+            const int row = warp * (2 * kHid) + 2 * j + half;
             w0[j].load(W + row * kHeadDim + col);
             w1[j].load(W + kHidden * kHeadDim + row * kHidden + col);
         }
-        w2.load(W + kHidden * kHeadDim + kHidden * kHidden + (warp * 2 + half) * kHidden + col);
 #pragma unroll
-        for (int j = 0; j < kRowLoads; ++j) {
-            const int row = warp * (2 * kRowLoads) + 2 * j + half;
-            b0[j] = __ldg(bias + row);
-            b1[j] = __ldg(bias + kHidden + row);
-        }
-        b2 = __ldg(bias + 2 * kHidden + warp * 2 + half);
+        for (int j = 0; j < kOut; ++j)
+            w2[j].load(W + kHidden * kHeadDim + kHidden * kHidden + (warp * (2 * kOut) + 2 * j + half) * kHidden + col);
+        b0 = __ldg(bias + warp * (2 * kHid) + 2 * spread_row<kHid>(sub) + half);
+        b1 = __ldg(bias + kHidden + warp * (2 * kHid) + 2 * spread_row<kHid>(sub) + half);
+        b2 = __ldg(bias + 2 * kHidden + warp * (2 * kOut) + 2 * spread_row<kOut>(sub) + half);
     }
 };
 
@@ -131,6 +180,13 @@ struct MlpSmem {
     float out[kCodeBits];
 };
 
+__device__ __forceinline__ void unpack_x8(const uint4 raw, float (&x)[8]) {
+    x[0] = bf16_lo(raw.x); x[1] = bf16_hi(raw.x);
+    x[2] = bf16_lo(raw.y); x[3] = bf16_hi(raw.y);
+    x[4] = bf16_lo(raw.z); x[5] = bf16_hi(raw.z);
+    x[6] = bf16_lo(raw.w); x[7] = bf16_hi(raw.w);
+}
+
 __device__ __forceinline__ void load_x8(const float* s, float (&x)[8]) {
     const float4 lo = *reinterpret_cast<const float4*>(s);
     const float4 hi = *reinterpret_cast<const float4*>(s + 4);
@@ -138,19 +194,19 @@ __device__ __forceinline__ void load_x8(const float* s, float (&x)[8]) {
     x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
 }
 
-// One hidden layer: every lane of a half-warp ends up with the kRowLoads row sums of its half;
-// lane j of the half then applies bias + SiLU to row j and stores it (one SiLU per lane).
-template <typename WT>
-__device__ __forceinline__ void hidden_layer(const Row8<WT> (&w)[kRowLoads], const float (&bias)[kRowLoads],
-                                             const float (&x)[8], float* dst, int warp, int lane) {
-    const int half = lane >> 4, sub = lane & 15;
-    float mine = 0.f;
+// One layer: the row sums of the warp's rows plus bias; a lane returns the one it ended up with.
+template <typename WT, int N>
+__device__ __forceinline__ float mlp_rows(const Row8<WT> (&w)[N], float bias, const float (&x)[8], int lane) {
+    float s[N];
 #pragma unroll
-    for (int j = 0; j < kRowLoads; ++j) {
-        const float s = half_warp_sum(w[j].dot(x)) + bias[j];
-        mine = sub == j ? s : mine;
-    }
-    if (sub < kRowLoads) dst[warp * (2 * kRowLoads) + 2 * sub + half] = silu(mine);
+    for (int j = 0; j < N; ++j) s[j] = w[j].dot(x);
+    return spread_sum<N>(s, lane & 15) + bias;
+}
+// stores a lane's row of a layer (one of the lanes that hold it)
+template <int N>
+__device__ __forceinline__ void mlp_store(float v, float* dst, int warp, int lane) {
+    const int half = lane >> 4, sub = lane & 15;
+    if (sub % (16 / N) == 0) dst[warp * (2 * N) + 2 * spread_row<N>(sub) + half] = v;
 }
 
 // Evaluates the MLP on one 128-element bf16 row, of which `raw` holds this lane's 8 elements
@@ -163,18 +219,14 @@ __device__ __forceinline__ void hidden_layer(const Row8<WT> (&w)[kRowLoads], con
 //
 // layers: 3 = all of W0, W1, W2; 2 = W0 then W2 (Linear-SiLU-Linear, hashattention_llama.py:112-120);
 // 1 = W2 alone (:121-127).
-template <typename WT, typename F>
-__device__ __forceinline__ void mlp_eval(const MlpRegs<WT>& r, const uint4 raw,
+template <typename WT, int kWarps, typename F>
+__device__ __forceinline__ void mlp_eval(const MlpRegs<WT, kWarps>& r, const uint4 raw,
                                          MlpSmem& sm, int warp, int lane, F&& between, int layers = 3) {
-    const int half = lane >> 4, col = (lane & 15) * 8;
+    constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
+    const int col = (lane & 15) * 8;
     float x[8];
-    {
-        x[0] = bf16_lo(raw.x); x[1] = bf16_hi(raw.x);
-        x[2] = bf16_lo(raw.y); x[3] = bf16_hi(raw.y);
-        x[4] = bf16_lo(raw.z); x[5] = bf16_hi(raw.z);
-        x[6] = bf16_lo(raw.w); x[7] = bf16_hi(raw.w);
-    }
-    if (layers >= 2) hidden_layer(r.w0, r.b0, x, sm.h0, warp, lane);
+    unpack_x8(raw, x);
+    if (layers >= 2) mlp_store<kHid>(silu(mlp_rows(r.w0, r.b0, x, lane)), sm.h0, warp, lane);
     between();
     if (layers >= 2) {
         __syncthreads();
@@ -183,53 +235,29 @@ __device__ __forceinline__ void mlp_eval(const MlpRegs<WT>& r, const uint4 raw,
         __syncthreads();  // no hidden layer separates this call's write of `out` from the previous call's readers
     }
     if (layers == 3) {
-        hidden_layer(r.w1, r.b1, x, sm.h1, warp, lane);
+        mlp_store<kHid>(silu(mlp_rows(r.w1, r.b1, x, lane)), sm.h1, warp, lane);
         __syncthreads();
         load_x8(sm.h1 + col, x);
     }
-    {
-        const float s = half_warp_sum(r.w2.dot(x)) + r.b2;
-        if ((lane & 15) == 0) sm.out[warp * 2 + half] = s;
-    }
+    mlp_store<kOut>(mlp_rows(r.w2, r.b2, x, lane), sm.out, warp, lane);
     __syncthreads();
 }
 
 // mlp_eval for two rows at once (`sm[0]`, `sm[1]`): the same weights in registers feed both rows, and the two
 // dependent chains (dot, shuffle reduction, SiLU, barrier) interleave, so the pair costs little more than one row.
-template <typename WT>
-__device__ __forceinline__ void hidden_layer2(const Row8<WT> (&w)[kRowLoads], const float (&bias)[kRowLoads],
-                                              const float (&xa)[8], const float (&xb)[8], float* da, float* db,
-                                              int warp, int lane) {
-    const int half = lane >> 4, sub = lane & 15;
-    float ma = 0.f, mb = 0.f;
-#pragma unroll
-    for (int j = 0; j < kRowLoads; ++j) {
-        const float sa = half_warp_sum(w[j].dot(xa)) + bias[j];
-        const float sb = half_warp_sum(w[j].dot(xb)) + bias[j];
-        ma = sub == j ? sa : ma;
-        mb = sub == j ? sb : mb;
-    }
-    if (sub < kRowLoads) {
-        da[warp * (2 * kRowLoads) + 2 * sub + half] = silu(ma);
-        db[warp * (2 * kRowLoads) + 2 * sub + half] = silu(mb);
-    }
-}
-
-__device__ __forceinline__ void unpack_x8(const uint4 raw, float (&x)[8]) {
-    x[0] = bf16_lo(raw.x); x[1] = bf16_hi(raw.x);
-    x[2] = bf16_lo(raw.y); x[3] = bf16_hi(raw.y);
-    x[4] = bf16_lo(raw.z); x[5] = bf16_hi(raw.z);
-    x[6] = bf16_lo(raw.w); x[7] = bf16_hi(raw.w);
-}
-
-template <typename WT, typename F>
-__device__ __forceinline__ void mlp_eval2(const MlpRegs<WT>& r, const uint4 raw_a, const uint4 raw_b,
+template <typename WT, int kWarps, typename F>
+__device__ __forceinline__ void mlp_eval2(const MlpRegs<WT, kWarps>& r, const uint4 raw_a, const uint4 raw_b,
                                           MlpSmem (&sm)[2], int warp, int lane, F&& between, int layers = 3) {
-    const int half = lane >> 4, col = (lane & 15) * 8;
+    constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
+    const int col = (lane & 15) * 8;
     float xa[8], xb[8];
     unpack_x8(raw_a, xa);
     unpack_x8(raw_b, xb);
-    if (layers >= 2) hidden_layer2(r.w0, r.b0, xa, xb, sm[0].h0, sm[1].h0, warp, lane);
+    if (layers >= 2) {
+        const float a = mlp_rows(r.w0, r.b0, xa, lane), b = mlp_rows(r.w0, r.b0, xb, lane);
+        mlp_store<kHid>(silu(a), sm[0].h0, warp, lane);
+        mlp_store<kHid>(silu(b), sm[1].h0, warp, lane);
+    }
     between();
     __syncthreads();
     if (layers >= 2) {
@@ -237,19 +265,16 @@ __device__ __forceinline__ void mlp_eval2(const MlpRegs<WT>& r, const uint4 raw_
         load_x8(sm[1].h0 + col, xb);
     }
     if (layers == 3) {
-        hidden_layer2(r.w1, r.b1, xa, xb, sm[0].h1, sm[1].h1, warp, lane);
+        const float a = mlp_rows(r.w1, r.b1, xa, lane), b = mlp_rows(r.w1, r.b1, xb, lane);
+        mlp_store<kHid>(silu(a), sm[0].h1, warp, lane);
+        mlp_store<kHid>(silu(b), sm[1].h1, warp, lane);
         __syncthreads();
         load_x8(sm[0].h1 + col, xa);
         load_x8(sm[1].h1 + col, xb);
     }
-    {
-        const float sa = half_warp_sum(r.w2.dot(xa)) + r.b2;
-        const float sb = half_warp_sum(r.w2.dot(xb)) + r.b2;
-        if ((lane & 15) == 0) {
-            sm[0].out[warp * 2 + half] = sa;
-            sm[1].out[warp * 2 + half] = sb;
-        }
-    }
+    const float a = mlp_rows(r.w2, r.b2, xa, lane), b = mlp_rows(r.w2, r.b2, xb, lane);
+    mlp_store<kOut>(a, sm[0].out, warp, lane);
+    mlp_store<kOut>(b, sm[1].out, warp, lane);
     __syncthreads();
 }
 
@@ -270,7 +295,7 @@ hash_decode_kernel(const HashDecodeParams p) {
 
     MlpRegs<WT> regs;
     regs.load(static_cast<const WT*>(p.w[side]) + (size_t)h * kMlpElems,
-              p.bias[side] + (size_t)h * kMlpBias, warp, lane >> 4, (lane & 15) * 8);
+              p.bias[side] + (size_t)h * kMlpBias, warp, lane);
     __shared__ MlpSmem sm[2];
 
     const int b_begin = blockIdx.z * p.batch_per_cta;
@@ -672,7 +697,7 @@ hash_prefill_simt_kernel(const HashPrefillParams p) {
 
     MlpRegs<WT> regs;
     regs.load(static_cast<const WT*>(p.wk) + (size_t)h * kMlpElems, p.bk + (size_t)h * kMlpBias,
-              warp, lane >> 4, (lane & 15) * 8);
+              warp, lane);
     __shared__ MlpSmem sm;
     pdl_wait();  // the keys may have been written by the kernel before this one
 
