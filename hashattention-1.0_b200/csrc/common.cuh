@@ -58,18 +58,6 @@ __host__ __device__ inline SeqRange seq_range(int S, int init_budget, int recent
     return r;
 }
 
-// Pages per score/select chunk: 4, 8 or 16 (the kernels are compiled for these), about
-// max_pages / 32 so that a sequence is cut into roughly 32 chunks.
-__host__ __device__ inline int chunk_pages_for(int max_pages) {
-    const int want = (max_pages + 31) / 32;
-    return want <= 4 ? 4 : (want <= 8 ? 8 : kMaxChunkPages);
-}
-
-__host__ __device__ inline int num_chunks_for(int max_pages) {
-    int cp = chunk_pages_for(max_pages);
-    return (max_pages + cp - 1) / cp;
-}
-
 __device__ __forceinline__ void report(int32_t* status, int code) {
     if (status != nullptr) atomicCAS(status, 0, code);
 }

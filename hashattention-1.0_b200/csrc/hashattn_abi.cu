@@ -110,24 +110,53 @@ AttSplit att_split_launch(const ha_shape_t* s, const ha_budget_t* b) {
 }
 
 // How a sequence is cut into chunks for scoring and selection: 4, 8 or 16 pages per chunk (the kernels are
-// compiled for these), about 32 chunks per sequence; small problems take smaller chunks (up to 64 per
-// sequence) until the scoring grid has two CTAs per SM.
+// compiled for these).
 struct Geometry {
     int chunk_pages, nchunks;
     int nslots;  // CTAs per (sequence, head) of select_attend_kernel: the chunks plus the two edge CTAs
 };
 
-Geometry geometry(const ha_shape_t* s) {
+Geometry geometry_of(const ha_shape_t* s, int chunk_pages) {
     Geometry g;
-    const int want = (s->max_pages + 31) / 32;
-    g.chunk_pages = want <= 4 ? 4 : (want <= 8 ? 8 : kMaxChunkPages);
-    const long long units = (long long)s->batch * s->num_kv_heads;
-    auto chunks = [&](int cp) { return (s->max_pages + cp - 1) / cp; };
-    while (g.chunk_pages > 4 && units * chunks(g.chunk_pages) < 2 * 148 && chunks(g.chunk_pages / 2) <= 64)
-        g.chunk_pages /= 2;
-    g.nchunks = chunks(g.chunk_pages);
+    g.chunk_pages = chunk_pages;
+    g.nchunks = (s->max_pages + chunk_pages - 1) / chunk_pages;
     g.nslots = g.nchunks + kSaEdgeSlots;
     return g;
+}
+
+// The cut is made for the attention that follows, whose CTAs own one chunk of one query head each:
+//   * about 128 attended rows per CTA. Fewer, and the fixed work of a CTA (ready word, classification, scan, partial)
+//     outweighs its gather: 32 sequences of 16K at a 1/32 budget take 146.9 us with 4-page chunks (32 rows), 117.7 with
+//     8, 104.6 with 16 (128 rows). Far more, and the rows all resident CTAs have asked L2 for no longer fit it:
+//     4 sequences of 128K at 1/4 take 329 us with 4 pages (256 rows), 412 with 8, 482 with 16; 32 x 16K at 1/8: 215 / 216
+//     / 282. In between nothing changes by more than 2 % (32 x 16K - 64K at 1/16: 345 us with 8 pages, 359 with 16).
+//   * at least two waves of CTAs (7 per SM), or the last wave and the uneven lists show: 8 x 16K at 1/32 takes 40.1 us
+//     with 16 pages (1536 CTAs), 38.5 with 8 (2560); 4 x 24K at 1/16 58.7 with 16, 50.5 with 8, 50.0 with 4. A sequence
+//     is not cut into more than 64 chunks for this, and a chunk is not larger than the longest sequence.
+Geometry geometry(const ha_shape_t* s, const ha_budget_t* b) {
+    const double tokens = (double)s->max_pages * kPage;
+    const double budget = b->heavy_budget > 1.0 ? b->heavy_budget : b->heavy_budget * tokens;
+    const double per_page = std::min(budget, (double)s->sel_stride) / s->max_pages;  // heavy rows of a head
+    const long long heads = (long long)s->batch * s->num_kv_heads * kGroup;
+    auto smaller_is_better = [&](int cp) {
+        const Geometry g = geometry_of(s, cp), half = geometry_of(s, cp / 2);
+        return per_page * cp > 192.0 || s->max_pages <= cp / 2 ||
+               (heads * g.nslots < 2 * 7 * 148 && half.nchunks <= 64);
+    };
+    int cp = kMaxChunkPages;
+    while (cp > 4 && smaller_is_better(cp)) cp /= 2;
+    return geometry_of(s, cp);
+}
+
+// The cut of the entry point whose scratch memory is built into the library: about 32 chunks per sequence, more of them
+// (up to 64) while the scoring grid has less than two CTAs per SM. Nothing is attended there, and the cut decides which
+// shapes fit the scratch memory.
+Geometry static_geometry(const ha_shape_t* s) {
+    const int want = (s->max_pages + 31) / 32;
+    int cp = want <= 4 ? 4 : (want <= 8 ? 8 : kMaxChunkPages);
+    const long long units = (long long)s->batch * s->num_kv_heads;
+    while (cp > 4 && units * geometry_of(s, cp).nchunks < 2 * 148 && geometry_of(s, cp / 2).nchunks <= 64) cp /= 2;
+    return geometry_of(s, cp);
 }
 
 struct Workspace {
@@ -145,7 +174,7 @@ size_t scores_bytes(const ha_shape_t* s, const Geometry& g) {
 }
 
 Workspace carve(const ha_shape_t* s, const ha_budget_t* b, void* base) {
-    const Geometry g = geometry(s);
+    const Geometry g = geometry(s, b);
     const size_t Hq = (size_t)s->num_kv_heads * kGroup, units = (size_t)s->batch * s->num_kv_heads;
     char* p = static_cast<char*>(base);
     Workspace w;
@@ -208,12 +237,12 @@ void prefer_carveout(K kernel, int kernel_id, int percent) {
 }
 
 // Scoring, histograms and the plan (score_hist_kernel) on the kv-heads [p.kvh0, p.kvh0 + nkvh).
-cudaError_t launch_score_hist(const ha_shape_t* shape, const SelectParams& p, int nkvh, cudaStream_t s) {
+cudaError_t launch_score_hist(const ha_shape_t* shape, int chunk_pages, const SelectParams& p, int nkvh, cudaStream_t s) {
     const dim3 grid(p.nchunks, nkvh, shape->batch);
     prefer_carveout(score_hist_kernel<1>, 0, 40);  // 5 CTAs x 13 KB
     prefer_carveout(score_hist_kernel<2>, 1, 40);
     prefer_carveout(score_hist_kernel<4>, 2, 40);
-    switch (geometry(shape).chunk_pages) {
+    switch (chunk_pages) {
         case 4: return launch(score_hist_kernel<1>, grid, dim3(kSelThreads), s, 1, p);
         case 8: return launch(score_hist_kernel<2>, grid, dim3(kSelThreads), s, 1, p);
         default: return launch(score_hist_kernel<4>, grid, dim3(kSelThreads), s, 1, p);
@@ -222,10 +251,9 @@ cudaError_t launch_score_hist(const ha_shape_t* shape, const SelectParams& p, in
 
 // Selection + attention (select_attend_kernel and the merge of its partials), or the selection alone, on the
 // query heads [p.h0, p.h0 + nheads).
-cudaError_t launch_select_attend(const ha_shape_t* shape, const SelectAttendParams& p, int nheads, bool gather,
-                                 cudaStream_t s) {
+cudaError_t launch_select_attend(const ha_shape_t* shape, int chunk_pages, const SelectAttendParams& p, int nheads,
+                                 bool gather, cudaStream_t s) {
     const dim3 grid(p.nslots, nheads, shape->batch);
-    const int chunk_pages = geometry(shape).chunk_pages;
     if (!gather) {
         switch (chunk_pages) {
             case 4: return launch(select_attend_kernel<1, false, 8>, grid, dim3(kSaThreads), s, 1, p);
@@ -279,7 +307,7 @@ bool use_cluster_select(const ha_shape_t* shape) {
 namespace ha {
 namespace {
 
-SelectParams select_params(const ha_shape_t* shape, const ha_budget_t* budget, const uint32_t* q_codes,
+SelectParams select_params(const ha_shape_t* shape, const ha_budget_t* budget, const Geometry& g, const uint32_t* q_codes,
                            const uint32_t* hash_pages, const int32_t* page_table, const int32_t* seq_lens,
                            int32_t* sel_idx, int32_t* sel_cnt, uint8_t* scores_dbg, int32_t* status,
                            uint32_t* hist, int32_t* plan, uint8_t* scores, uint32_t* arrive, int32_t* sel_rows,
@@ -304,7 +332,7 @@ SelectParams select_params(const ha_shape_t* shape, const ha_budget_t* budget, c
     p.max_pages = shape->max_pages;
     p.num_pages = shape->num_pages;
     p.sel_stride = shape->sel_stride;
-    p.nchunks = geometry(shape).nchunks;
+    p.nchunks = g.nchunks;
     p.kvh0 = 0;
     p.init_budget = budget->init_budget;
     p.recent_budget = budget->recent_budget;
@@ -316,12 +344,11 @@ SelectParams select_params(const ha_shape_t* shape, const ha_budget_t* budget, c
 }
 
 // The attention side (q, pools, out) may be null when only the selection is run.
-SelectAttendParams select_attend_params(const ha_shape_t* shape, const ha_budget_t* budget, const int32_t* plan,
+SelectAttendParams select_attend_params(const ha_shape_t* shape, const ha_budget_t* budget, const Geometry& g, const int32_t* plan,
                                         const uint8_t* scores, float* partials, int32_t* sel_idx, const void* q,
                                         const void* k_pages, const void* v_pages, const int32_t* page_table,
                                         const int32_t* seq_lens, const int32_t* budget_lens, float sm_scale, void* out,
                                         int32_t* status, int32_t* status_out) {
-    const Geometry g = geometry(shape);
     SelectAttendParams p;
     p.plan = plan;
     p.scores = scores;
@@ -797,7 +824,8 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     const Workspace w = carve(shape, budget, workspace);
     if (workspace_bytes < w.bytes) return HA_ERR_WORKSPACE;
 
-    SelectParams p = select_params(shape, budget, q_codes, hash_pages, page_table, seq_lens, sel_idx, sel_cnt,
+    const Geometry g = geometry(shape, budget);
+    SelectParams p = select_params(shape, budget, g, q_codes, hash_pages, page_table, seq_lens, sel_idx, sel_cnt,
                                    scores_dbg, status, w.hist, w.plan, w.scores, w.arrive, w.sel_rows, budget_lens);
     // handover: the caller launches the selection right behind this call; it then takes each unit's plan as soon as
     // that unit is ready instead of waiting for the whole scoring grid
@@ -812,13 +840,13 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
             : launch(score_select_cluster_kernel<2>, cgrid, dim3(kClThreads), s, kClCtas, p);
         return e == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
     }
-    if (launch_score_hist(shape, p, shape->num_kv_heads, s) != cudaSuccess) return HA_ERR_LAUNCH;
+    if (launch_score_hist(shape, g.chunk_pages, p, shape->num_kv_heads, s) != cudaSuccess) return HA_ERR_LAUNCH;
     if (plan_only) return HA_OK;
-    SelectAttendParams sa = select_attend_params(shape, budget, w.plan, w.scores, w.partials, sel_idx, nullptr,
+    SelectAttendParams sa = select_attend_params(shape, budget, g, w.plan, w.scores, w.partials, sel_idx, nullptr,
                                                  nullptr, nullptr, page_table, seq_lens, budget_lens, 1.0f,
                                                  nullptr, status, nullptr);
     if (ho != 0) sa.ready = reinterpret_cast<int32_t*>(w.arrive);
-    return launch_select_attend(shape, sa, shape->num_kv_heads * kGroup, false, s) == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
+    return launch_select_attend(shape, g.chunk_pages, sa, shape->num_kv_heads * kGroup, false, s) == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
 }
 
 // The selection + attention stage on the plan and score bytes a scoring call left in the workspace.
@@ -837,11 +865,12 @@ static int select_attend_impl(const ha_shape_t* shape, const ha_budget_t* budget
     if (workspace == nullptr) return HA_ERR_WORKSPACE;
     const Workspace w = carve(shape, budget, workspace);
     if (workspace_bytes < w.bytes) return HA_ERR_WORKSPACE;
-    SelectAttendParams sa = select_attend_params(shape, budget, w.plan, w.scores, w.partials, sel_idx, q, k_pages,
+    const Geometry g = geometry(shape, budget);
+    SelectAttendParams sa = select_attend_params(shape, budget, g, w.plan, w.scores, w.partials, sel_idx, q, k_pages,
                                                  v_pages, page_table, seq_lens, budget_lens, sm_scale, out,
                                                  status, status_out);
     if (handover) sa.ready = reinterpret_cast<int32_t*>(w.arrive);  // (the scoring call in front was told the same)
-    return launch_select_attend(shape, sa, shape->num_kv_heads * kGroup, true, static_cast<cudaStream_t>(stream)) ==
+    return launch_select_attend(shape, g.chunk_pages, sa, shape->num_kv_heads * kGroup, true, static_cast<cudaStream_t>(stream)) ==
                    cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
 }
 
@@ -1101,7 +1130,7 @@ struct StaticScratch {
 };
 
 StaticScratch carve_static(const ha_shape_t* s, void* base) {
-    const ha::Geometry g = ha::geometry(s);
+    const ha::Geometry g = ha::static_geometry(s);
     const size_t units = (size_t)s->batch * s->num_kv_heads;
     char* p = static_cast<char*>(base);
     StaticScratch w;
@@ -1164,13 +1193,14 @@ int ha_score_select_static(const ha_shape_t* shape, const ha_budget_t* budget,
     // Every other word a kernel reads was written earlier in the same call.
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(w.arrive, 0, w.arrive_bytes, s) != cudaSuccess) return HA_ERR_LAUNCH;
-    const SelectParams p = select_params(shape, budget, q_codes, hash_pages, page_table, seq_lens, sel_idx, sel_cnt,
+    const ha::Geometry g = ha::static_geometry(shape);
+    const SelectParams p = select_params(shape, budget, g, q_codes, hash_pages, page_table, seq_lens, sel_idx, sel_cnt,
                                          nullptr, status, w.hist, w.plan, w.scores, w.arrive, nullptr);
-    if (launch_score_hist(shape, p, shape->num_kv_heads, s) != cudaSuccess) return HA_ERR_LAUNCH;
-    const SelectAttendParams sa = select_attend_params(shape, budget, w.plan, w.scores, nullptr, sel_idx, nullptr,
+    if (launch_score_hist(shape, g.chunk_pages, p, shape->num_kv_heads, s) != cudaSuccess) return HA_ERR_LAUNCH;
+    const SelectAttendParams sa = select_attend_params(shape, budget, g, w.plan, w.scores, nullptr, sel_idx, nullptr,
                                                        nullptr, nullptr, page_table, seq_lens, nullptr, 1.0f, nullptr,
                                                        status, nullptr);
-    return launch_select_attend(shape, sa, shape->num_kv_heads * kGroup, false, s) == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
+    return launch_select_attend(shape, g.chunk_pages, sa, shape->num_kv_heads * kGroup, false, s) == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
 }
 
 }  // extern "C"

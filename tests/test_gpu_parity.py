@@ -507,6 +507,45 @@ def test_long_sequence_selection(device, S):
     run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 32, 128), shuffle_seed=2)
 
 
+def test_more_than_64_chunks_per_sequence(device):
+    """A quarter of 70,000 tokens is attended: 4-page chunks, 69 of them, which the plan sweeps in two passes."""
+    usa = synthetic.make_usa(4, 128, 4, True)
+    inp = synthetic.make_decode_inputs(106, [70000], 4, 1)
+    run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 4, 128), shuffle_seed=2)
+
+
+@pytest.mark.parametrize("lens,heavy", [
+    ([2817, 4095, 1, 257, 2049, 3000] * 4, 1.0 / 32),       # 16-page chunks: at most one per sequence
+    ([4096, 4097, 9000, 130, 8192, 2047] * 3, 1.0 / 32),    # ... up to three, lengths at their edges
+    ([4096, 4097, 9000, 2048, 8193, 255] * 2, 1.0 / 16),    # 8-page chunks
+])
+def test_large_batch_in_large_chunks_equals_its_sequences_alone(device, lib_option, lens, heavy):
+    """A large batch is cut into large chunks, one sequence of it into 4-page ones (which the cases above compare with the
+    oracle): both select the same sets, and the outputs agree to rounding (partials merged in another order)."""
+    Hkv = 8
+    lib_option("cluster_select", 0)
+    cache = ha.PagedHashKVCache(len(lens), Hkv, max(lens), device, shuffle_seed=5)
+    synthetic.fill_cache_on_device(cache, lens, seed=5)
+    usa, budget = synthetic.make_usa(4 * Hkv, 128, 5, True), ha.Budget(128, heavy, 64)
+    ctx = ha.SparseDecodeContext(cache, budget, usa.packed(device))
+    ctx.hash_prefill()
+    gen = torch.Generator(device=device).manual_seed(5)
+    q, k, v = (torch.randn(len(lens), n, 128, generator=gen, device=device).bfloat16() for n in (4 * Hkv, Hkv, Hkv))
+    out = ctx.decode_step(q, k, v).float().cpu()
+    ctx.check_status()
+    for b in range(6):
+        one = copy.copy(cache)
+        one.batch, one.page_table, one.seq_lens = 1, cache.page_table[b:b + 1].contiguous(), cache.seq_lens[b:b + 1].contiguous()
+        alone = ha.SparseDecodeContext(one, budget, usa.packed(device))
+        ref = alone.decode_step(q[b:b + 1].contiguous(), k[b:b + 1].contiguous(), v[b:b + 1].contiguous()).float().cpu()
+        alone.check_status()
+        assert torch.equal(ctx.sel_cnt[b], alone.sel_cnt[0])
+        for h in range(4 * Hkv):
+            assert torch.equal(heavy_from_device(ctx, b, h), heavy_from_device(alone, 0, h)), (b, h)
+        ok, max_abs, rel = helpers.att_close(out[b:b + 1], ref)
+        assert ok, (b, max_abs, rel)
+
+
 def test_selection_alone_through_the_scoring_kernel_and_the_select_only_kernel(device):
     """S = 40,000 through the workspace-free entry point, which always runs the scoring kernel and the
     selection-only build of the fused kernel (two rounds per scoring CTA here), against the oracle on the
