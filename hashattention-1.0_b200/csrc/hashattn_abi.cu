@@ -285,7 +285,7 @@ cudaError_t launch_select_attend(const ha_shape_t* shape, int chunk_pages, const
         }
     }
     if (e != cudaSuccess) return e;
-    return launch(select_attend_merge_kernel, dim3(nheads, shape->batch), dim3(kMergeThreads), s, 1, p, chunk_pages * kPage);
+    return launch(select_attend_merge_kernel, dim3(nheads, shape->batch), dim3(32 * merge_warps(p.nslots)), s, 1, p, chunk_pages * kPage);
 }
 
 // One cluster kernel scores and selects in a single pass when the sequences are short and there are at

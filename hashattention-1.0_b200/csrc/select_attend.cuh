@@ -454,19 +454,21 @@ __global__ void __launch_bounds__(kSaThreads, kMinCtas) select_attend_kernel(con
 }
 
 // Log-sum-exp merge of the partials select_attend_kernel left for one (sequence, head): the partials of the CTAs
-// that had a chunk (those below the sequence length) and of the two edge CTAs. 512 threads: thread = (output
-// dimension, one of 4 slices of the partials), so that up to 68 partials are fetched in one trip with at most
-// 17 x 3 loads per thread in flight; the slices are combined in shared memory.
-constexpr int kMergeSlices = 4;
-constexpr int kMergeThreads = kHeadDim * kMergeSlices;
-constexpr int kMergeBatch = 17;
+// that had a chunk (those below the sequence length) and of the two edge CTAs. A warp takes every warps-th partial, four
+// dimensions per lane, kMergeBatch of them in one trip; the warps are combined in shared memory. 4 warps where the
+// partials fit one trip (kMergeBatch each), else 8, for the sake of the registers: at 1024 heads a CTA of 512 threads
+// with 110 registers each ran one per SM and took seven waves (step of 32 x 16K at a 1/32 budget: 104.7 -> 93.9 us;
+// 32 x 40K at 1/16: 282 -> 271; with 128 heads unchanged).
+constexpr int kMergeMaxWarps = 8;
+constexpr int kMergeBatch = 9;
+inline int merge_warps(int nslots) { return nslots <= 4 * kMergeBatch ? 4 : kMergeMaxWarps; }
 
-__global__ void __launch_bounds__(kMergeThreads) select_attend_merge_kernel(const SelectAttendParams p, int chunk_tokens) {
+__global__ void __launch_bounds__(32 * kMergeMaxWarps, 3) select_attend_merge_kernel(const SelectAttendParams p, int chunk_tokens) {
     const int h = p.h0 + blockIdx.x, b = blockIdx.y;
     const int Hq = p.Hkv * kGroup;
-    const int tid = threadIdx.x, d = tid % kHeadDim, slice = tid / kHeadDim;
-    __shared__ float s_m[kMergeSlices], s_l[kMergeSlices];
-    __shared__ float s_a[kMergeSlices][kHeadDim];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    __shared__ float s_m[kMergeMaxWarps], s_l[kMergeMaxWarps];
+    __shared__ float2 s_a[kMergeMaxWarps][kHeadDim / 2];
     const int S = p.seq_lens[b];
     const bool ok = S >= 1 && S <= p.max_pages * kPage;
     const int nparts = kSaEdgeSlots + (S + chunk_tokens - 1) / chunk_tokens;
@@ -477,50 +479,56 @@ __global__ void __launch_bounds__(kMergeThreads) select_attend_merge_kernel(cons
     if (!ok) return;
 
     const float* base = p.partials + ((size_t)b * Hq + h) * p.nslots * kPartStride;
-    // this slice's partials: j = slice + 4 i
-    const int mine = (nparts - slice + kMergeSlices - 1) / kMergeSlices;
-    float Mg = -INFINITY, Lg = 0.f, Ag = 0.f;
+    // this warp's partials: j = warp + warps * i; lane: dimensions 2 lane, 2 lane + 1, 64 + 2 lane, 65 + 2 lane
+    const int mine = (nparts - warp + warps - 1) / warps;
+    float Mg = -INFINITY, Lg = 0.f;
+    float2 Aa = make_float2(0.f, 0.f), Ab = Aa;
+    static_assert(kPartStride % 2 == 0, "8-byte loads of a partial");
     for (int i0 = 0; i0 < mine; i0 += kMergeBatch) {
         const int n = min(kMergeBatch, mine - i0);
-        float ms[kMergeBatch], ls[kMergeBatch], as[kMergeBatch];
+        float2 ml[kMergeBatch], aa[kMergeBatch], ab[kMergeBatch];
 #pragma unroll
         for (int j = 0; j < kMergeBatch; ++j) {
-            const float* ps = base + (size_t)(slice + kMergeSlices * (i0 + min(j, n - 1))) * kPartStride;
-            ms[j] = __ldcg(ps);
-            ls[j] = __ldcg(ps + 1);
-            as[j] = __ldcg(ps + 2 + d);
+            const float2* ps = reinterpret_cast<const float2*>(base + (size_t)(warp + warps * (i0 + min(j, n - 1))) * kPartStride);
+            ml[j] = __ldcg(ps);
+            aa[j] = __ldcg(ps + 1 + lane);
+            ab[j] = __ldcg(ps + 33 + lane);
         }
         float mb = Mg;
 #pragma unroll
-        for (int j = 0; j < kMergeBatch; ++j) mb = fmaxf(mb, j < n ? ms[j] : -INFINITY);
+        for (int j = 0; j < kMergeBatch; ++j) mb = fmaxf(mb, j < n ? ml[j].x : -INFINITY);
         const float rescale = Mg == -INFINITY ? 0.f : fast_exp2(Mg - mb);
         Mg = mb;
         Lg *= rescale;
-        Ag *= rescale;
+        Aa.x *= rescale; Aa.y *= rescale; Ab.x *= rescale; Ab.y *= rescale;
 #pragma unroll
         for (int j = 0; j < kMergeBatch; ++j) {
-            const float f = (j < n && ms[j] != -INFINITY) ? fast_exp2(ms[j] - Mg) : 0.f;
-            Lg = fmaf(ls[j], f, Lg);
-            Ag = fmaf(as[j], f, Ag);
+            const float f = (j < n && ml[j].x != -INFINITY) ? fast_exp2(ml[j].x - Mg) : 0.f;
+            Lg = fmaf(ml[j].y, f, Lg);
+            Aa.x = fmaf(aa[j].x, f, Aa.x); Aa.y = fmaf(aa[j].y, f, Aa.y);
+            Ab.x = fmaf(ab[j].x, f, Ab.x); Ab.y = fmaf(ab[j].y, f, Ab.y);
         }
     }
-    if (d == 0) {
-        s_m[slice] = Mg;
-        s_l[slice] = Lg;
+    if (lane == 0) {
+        s_m[warp] = Mg;
+        s_l[warp] = Lg;
     }
-    s_a[slice][d] = Ag;
+    s_a[warp][lane] = Aa;
+    s_a[warp][32 + lane] = Ab;
     __syncthreads();
-    if (slice != 0) return;
-    float M = -INFINITY, L = 0.f, A = 0.f;
-#pragma unroll
-    for (int w = 0; w < kMergeSlices; ++w) M = fmaxf(M, s_m[w]);
-#pragma unroll
-    for (int w = 0; w < kMergeSlices; ++w) {
+    if (warp >= 2) return;  // 64 threads, two dimensions each
+    float M = -INFINITY, L = 0.f;
+    float2 A = make_float2(0.f, 0.f);
+    for (int w = 0; w < warps; ++w) M = fmaxf(M, s_m[w]);
+    for (int w = 0; w < warps; ++w) {
         const float f = s_m[w] == -INFINITY ? 0.f : fast_exp2(s_m[w] - M);
         L = fmaf(s_l[w], f, L);
-        A = fmaf(s_a[w][d], f, A);
+        A.x = fmaf(s_a[w][tid].x, f, A.x);
+        A.y = fmaf(s_a[w][tid].y, f, A.y);
     }
-    p.out[((size_t)b * Hq + h) * kHeadDim + d] = __float2bfloat16_rn(L > 0.f ? A / L : 0.f);
+    __nv_bfloat16* out = p.out + ((size_t)b * Hq + h) * kHeadDim + 2 * tid;  // (aligned to one element: two stores)
+    out[0] = __float2bfloat16_rn(L > 0.f ? A.x / L : 0.f);
+    out[1] = __float2bfloat16_rn(L > 0.f ? A.y / L : 0.f);
 }
 
 }  // namespace ha

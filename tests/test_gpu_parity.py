@@ -507,10 +507,12 @@ def test_long_sequence_selection(device, S):
     run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 32, 128), shuffle_seed=2)
 
 
-def test_more_than_64_chunks_per_sequence(device):
-    """A quarter of 70,000 tokens is attended: 4-page chunks, 69 of them, which the plan sweeps in two passes."""
+@pytest.mark.parametrize("S", [70000, 80000])
+def test_more_than_64_chunks_per_sequence(device, S):
+    """A quarter of the tokens is attended: 4-page chunks, 69 or 79 of them, which the plan sweeps in two passes; their
+    partials (and the two edge ones) take the merge one or two trips of 72."""
     usa = synthetic.make_usa(4, 128, 4, True)
-    inp = synthetic.make_decode_inputs(106, [70000], 4, 1)
+    inp = synthetic.make_decode_inputs(106, [S], 4, 1)
     run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 4, 128), shuffle_seed=2)
 
 
