@@ -835,7 +835,9 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     const long long max_tokens = (long long)shape->max_pages * kPage;
     if (!plan_only && use_cluster_select(shape)) {
         const dim3 cgrid(kClCtas, shape->num_kv_heads, shape->batch);
-        const cudaError_t e = max_tokens <= kClRoundTokens
+        const cudaError_t e = max_tokens <= kCsMaxTokens
+            ? launch(score_select_short_kernel, cgrid, dim3(kCsThreads), s, kClCtas, p)
+            : max_tokens <= kClRoundTokens
             ? launch(score_select_cluster_kernel<1>, cgrid, dim3(kClThreads), s, kClCtas, p)
             : launch(score_select_cluster_kernel<2>, cgrid, dim3(kClThreads), s, kClCtas, p);
         return e == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;

@@ -548,6 +548,16 @@ def test_large_batch_in_large_chunks_equals_its_sequences_alone(device, lib_opti
         assert ok, (b, max_abs, rel)
 
 
+@pytest.mark.parametrize("lens", [[1024, 1025], [127, 128], [2047, 2049], [16384], [16385]])
+def test_cluster_selection_at_the_edges_of_its_parts(device, lens):
+    """Sequences around whole blocks of the eight CTAs of a cluster, the largest one the short-sequence kernel takes and
+    the smallest one beyond it."""
+    usa = synthetic.make_usa(8, 128, 4, True)
+    inp = synthetic.make_decode_inputs(107, lens, 8, 2)
+    _, _, ctx, _ = run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(16, 1.0 / 16, 16), shuffle_seed=2)
+    assert "cluster" in ctx.step_path()
+
+
 def test_selection_alone_through_the_scoring_kernel_and_the_select_only_kernel(device):
     """S = 40,000 through the workspace-free entry point, which always runs the scoring kernel and the
     selection-only build of the fused kernel (two rounds per scoring CTA here), against the oracle on the
