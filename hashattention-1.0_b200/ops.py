@@ -7,6 +7,7 @@ A non-zero library status raises ``RuntimeError``. There is no torch or CPU fall
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 from dataclasses import dataclass
@@ -55,7 +56,7 @@ def _check(t: torch.Tensor, name: str, dtype: torch.dtype, shape, device) -> Non
         raise ValueError(f"{name} must be a tensor")
     if t.dtype != dtype:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
-    if tuple(t.shape) != tuple(shape):
+    if t.shape != shape and tuple(t.shape) != tuple(shape):
         raise ValueError(f"{name} should be of size {tuple(shape)}, but is {tuple(t.shape)}")
     if t.device != device:
         raise ValueError(f"{name} must live on {device}, got {t.device}")
@@ -66,6 +67,14 @@ def _check(t: torch.Tensor, name: str, dtype: torch.dtype, shape, device) -> Non
 def _raise_on(rc: int, what: str) -> None:
     if rc != _lib.HA_OK:
         raise RuntimeError(f"{what} failed: {_lib.status_str(rc)} (status {rc})")
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def on_device(device):
+    """``torch.cuda.device(device)``, or nothing where that device is the current one already (1 us less per call)."""
+    return _SAME_DEVICE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _stream_ptr(device) -> int:
@@ -176,7 +185,7 @@ class SparseDecodeContext:
         if preact_dbg is not None:
             _check(preact_dbg, "preact_dbg", torch.float32, (self.batch, 2, self.num_q_heads, 32), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_hash_decode"):
+        with on_device(self.device), _call_range("ha_hash_decode"):
             rc = self.lib.ha_hash_decode(
                 self.shape, self.c_weights, q.data_ptr(), k_new.data_ptr() if k_new is not None else None,
                 v_new.data_ptr() if v_new is not None else None, c.k_pages.data_ptr(), c.v_pages.data_ptr(),
@@ -191,7 +200,7 @@ class SparseDecodeContext:
         if first_token is not None:
             _check(first_token, "first_token", torch.int32, (self.batch,), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_hash_prefill"):
+        with on_device(self.device), _call_range("ha_hash_prefill"):
             rc = self.lib.ha_hash_prefill(
                 self.shape, self.c_weights, c.k_pages.data_ptr(), c.hash_pages.data_ptr(), c.page_table.data_ptr(),
                 c.seq_lens.data_ptr(), first_token.data_ptr() if first_token is not None else None,
@@ -206,7 +215,7 @@ class SparseDecodeContext:
             _check(scores_dbg, "scores_dbg", torch.uint8,
                    (self.batch, self.num_q_heads, self.cache.max_pages * PAGE), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_score_select"):
+        with on_device(self.device), _call_range("ha_score_select"):
             rc = self.lib.ha_score_select(
                 self.shape, self.c_budget, q_codes.data_ptr(), c.hash_pages.data_ptr(), c.page_table.data_ptr(),
                 c.seq_lens.data_ptr(), self.sel_idx.data_ptr(), self.sel_cnt.data_ptr(),
@@ -221,7 +230,7 @@ class SparseDecodeContext:
         q_codes = self.q_codes if q_codes is None else q_codes
         _check(q_codes, "q_codes", torch.int32, (self.batch, self.num_q_heads), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_score_plan"):
+        with on_device(self.device), _call_range("ha_score_plan"):
             rc = self.lib.ha_score_plan(
                 self.shape, self.c_budget, q_codes.data_ptr(), c.hash_pages.data_ptr(), c.page_table.data_ptr(),
                 c.seq_lens.data_ptr(), self.sel_cnt.data_ptr(), self.workspace.data_ptr(), self.workspace_bytes,
@@ -236,7 +245,7 @@ class SparseDecodeContext:
         out = torch.empty_like(q) if out is None else out
         _check(out, "out", torch.bfloat16, (self.batch, self.num_q_heads, HEAD_DIM), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_select_attend"):
+        with on_device(self.device), _call_range("ha_select_attend"):
             rc = self.lib.ha_select_attend(
                 self.shape, self.c_budget, q.data_ptr(), c.k_pages.data_ptr(), c.v_pages.data_ptr(),
                 c.page_table.data_ptr(), c.seq_lens.data_ptr(), self.sel_idx.data_ptr(), self.sm_scale,
@@ -259,7 +268,7 @@ class SparseDecodeContext:
         q_codes = self.q_codes if q_codes is None else q_codes
         _check(q_codes, "q_codes", torch.int32, (self.batch, self.num_q_heads), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_score_select_static"):
+        with on_device(self.device), _call_range("ha_score_select_static"):
             rc = self.lib.ha_score_select_static(
                 self.shape, self.c_budget, q_codes.data_ptr(), c.hash_pages.data_ptr(), c.page_table.data_ptr(),
                 c.seq_lens.data_ptr(), self.sel_idx.data_ptr(), self.sel_cnt.data_ptr(), self.status.data_ptr(),
@@ -277,7 +286,7 @@ class SparseDecodeContext:
         _check(sel_idx, "sel_idx", torch.int32, (self.batch, self.num_q_heads, self.sel_stride), self.device)
         _check(sel_cnt, "sel_cnt", torch.int32, (self.batch, self.num_q_heads), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_sparse_decode"):
+        with on_device(self.device), _call_range("ha_sparse_decode"):
             rc = self.lib.ha_sparse_decode(
                 self.shape, self.c_budget, q.data_ptr(), c.k_pages.data_ptr(), c.v_pages.data_ptr(),
                 c.page_table.data_ptr(), c.seq_lens.data_ptr(), sel_idx.data_ptr(), sel_cnt.data_ptr(),
@@ -301,7 +310,7 @@ class SparseDecodeContext:
             raise ValueError("v_new is required")
         out = torch.empty_like(q) if out is None else out
         _check(out, "out", torch.bfloat16, (self.batch, self.num_q_heads, HEAD_DIM), self.device)
-        with torch.cuda.device(self.device), _call_range("ha_decode_step_rows"):
+        with on_device(self.device), _call_range("ha_decode_step_rows"):
             rc = self.lib.ha_decode_step_rows(
                 self.shape, self.c_budget, self.c_weights, q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(),
                 c.k_pages.data_ptr(), c.v_pages.data_ptr(), c.hash_pages.data_ptr(), c.page_table.data_ptr(),
@@ -318,7 +327,7 @@ class SparseDecodeContext:
         out = torch.empty_like(q) if out is None else out
         _check(out, "out", torch.bfloat16, (self.batch, self.num_q_heads, HEAD_DIM), self.device)
         c = self.cache
-        with torch.cuda.device(self.device), _call_range("ha_decode_step"):
+        with on_device(self.device), _call_range("ha_decode_step"):
             rc = self.lib.ha_decode_step(
                 self.shape, self.c_budget, self.c_weights, q.data_ptr(), k_new.data_ptr(),
                 v_new.data_ptr() if v_new is not None else None, c.k_pages.data_ptr(), c.v_pages.data_ptr(),

@@ -16,8 +16,10 @@ import torch
 
 from . import _lib
 from .cache import GROUP, HEAD_DIM, PAGE
+from .ops import on_device
 
-_MUTATED = ("k_pages", "v_pages", "hash_pages", "q_codes", "sel_idx", "sel_cnt", "workspace", "status", "out")
+_TENSORS = ("q", "k_new", "v_new", "k_pages", "v_pages", "hash_pages", "page_table", "seq_lens", "wq", "bq", "wk", "bk",
+            "q_codes", "sel_idx", "sel_cnt", "workspace", "status", "out")
 
 
 def _shape_of(q, k_new, k_pages, page_table, sel_idx) -> _lib.HaShape:
@@ -31,27 +33,57 @@ def _shape_of(q, k_new, k_pages, page_table, sel_idx) -> _lib.HaShape:
                         sel_idx.shape[2])
 
 
-@torch.library.custom_op("hashattn::decode_step", mutates_args=_MUTATED, device_types="cuda")
-def decode_step(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
-                k_pages: torch.Tensor, v_pages: torch.Tensor, hash_pages: torch.Tensor,
-                page_table: torch.Tensor, seq_lens: torch.Tensor,
-                wq: torch.Tensor, bq: torch.Tensor, wk: torch.Tensor, bk: torch.Tensor,
-                q_codes: torch.Tensor, sel_idx: torch.Tensor, sel_cnt: torch.Tensor,
-                workspace: torch.Tensor, status: torch.Tensor, out: torch.Tensor,
-                init_budget: int, recent_budget: int, heavy_budget: float, sm_scale: float,
-                eval_mode: int = 0, retrieve_depth: int = 0, num_hash_layers: int = 3) -> None:
+# The operator is defined by its schema and two kernels instead of torch.library.custom_op, whose three Python layers per
+# call (autograd, version counters, backend) took 30 us of host time for these 25 arguments - more than the step takes on
+# the GPU - against 13 us here; what they did is kept: see _autograd and the end of _decode_step_cuda.
+if "_LIB" in globals():  # the module is being reloaded
+    globals()["_LIB"]._destroy()
+_LIB = torch.library.Library("hashattn", "DEF")
+_LIB.define(
+    "decode_step(Tensor q, Tensor k_new, Tensor v_new, Tensor(a3!) k_pages, Tensor(a4!) v_pages, Tensor(a5!) hash_pages, "
+    "Tensor page_table, Tensor seq_lens, Tensor wq, Tensor bq, Tensor wk, Tensor bk, Tensor(a12!) q_codes, "
+    "Tensor(a13!) sel_idx, Tensor(a14!) sel_cnt, Tensor(a15!) workspace, Tensor(a16!) status, Tensor(a17!) out, "
+    "SymInt init_budget, SymInt recent_budget, float heavy_budget, float sm_scale, SymInt eval_mode=0, "
+    "SymInt retrieve_depth=0, SymInt num_hash_layers=3) -> ()", tags=(torch.Tag.pt2_compliant_tag,))
+decode_step = torch.ops.hashattn.decode_step.default
+
+
+class _NoFormula(torch.autograd.Function):
+    """The step below autograd, without a backward: nothing it writes is connected to its inputs, and function transforms
+    (torch.func.grad and the like) are refused, since there is no setup_context."""
+
+    @staticmethod
+    def forward(ctx, *args):
+        with torch._C._AutoDispatchBelowAutograd():
+            return decode_step(*args)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        raise RuntimeError("Trying to backward through hashattn::decode_step but no autograd formula was registered.")
+
+
+def _autograd(keyset, *args):
+    if torch.is_grad_enabled() and any([a.requires_grad for a in args[:len(_TENSORS)]]):
+        return _NoFormula.apply(*args)
+    return decode_step.redispatch(keyset & torch._C._after_autograd_keyset, *args)
+
+
+def _decode_step_cuda(q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk,
+                      q_codes, sel_idx, sel_cnt, workspace, status, out,
+                      init_budget, recent_budget, heavy_budget, sm_scale, eval_mode=0, retrieve_depth=0,
+                      num_hash_layers=3) -> None:
     lib = _lib.load()
-    tensors = dict(q=q, k_new=k_new, v_new=v_new, k_pages=k_pages, v_pages=v_pages, hash_pages=hash_pages,
-                   page_table=page_table, seq_lens=seq_lens, wq=wq, bq=bq, wk=wk, bk=bk, q_codes=q_codes,
-                   sel_idx=sel_idx, sel_cnt=sel_cnt, workspace=workspace, status=status, out=out)
-    for name, t in tensors.items():
-        if t.device != q.device:
-            raise ValueError(f"{name} must live on {q.device}, got {t.device}")
+    device = q.device
+    tensors = (q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk, q_codes, sel_idx, sel_cnt,
+               workspace, status, out)
+    for i, t in enumerate(tensors):
+        if t.device != device:
+            raise ValueError(f"{_TENSORS[i]} must live on {device}, got {t.device}")
         if not t.is_contiguous():
-            raise ValueError(f"{name} must be contiguous")
-    for name in ("q", "k_new", "v_new", "k_pages", "v_pages", "out"):
-        if tensors[name].dtype != torch.bfloat16:
-            raise ValueError(f"{name} must be torch.bfloat16, got {tensors[name].dtype}")
+            raise ValueError(f"{_TENSORS[i]} must be contiguous")
+    for i in (0, 1, 2, 3, 4, 17):
+        if tensors[i].dtype != torch.bfloat16:
+            raise ValueError(f"{_TENSORS[i]} must be torch.bfloat16, got {tensors[i].dtype}")
     if wq.dtype != wk.dtype or wq.dtype not in (torch.bfloat16, torch.float32):
         raise ValueError("hash weights must both be bfloat16 or both float32")
     shape = _shape_of(q, k_new, k_pages, page_table, sel_idx)
@@ -60,26 +92,34 @@ def decode_step(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
     weights = _lib.HaHashWeights(wq.data_ptr(), bq.data_ptr(), wk.data_ptr(), bk.data_ptr(),
                                  _lib.HA_WEIGHTS_BF16 if wq.dtype == torch.bfloat16 else _lib.HA_WEIGHTS_F32,
                                  int(num_hash_layers))
-    need = int(lib.ha_workspace_bytes(shape, budget))
-    if need == 0 or workspace.numel() * workspace.element_size() < need:
-        raise ValueError(f"workspace holds {workspace.numel() * workspace.element_size()} bytes, the step needs {need}")
-    with torch.cuda.device(q.device):
+    need, have = int(lib.ha_workspace_bytes(shape, budget)), workspace.numel() * workspace.element_size()
+    if need == 0 or have < need:
+        raise ValueError(f"workspace holds {have} bytes, the step needs {need}")
+    with on_device(device):
         rc = lib.ha_decode_step(shape, budget, weights, q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(),
                                 k_pages.data_ptr(), v_pages.data_ptr(), hash_pages.data_ptr(), page_table.data_ptr(),
                                 seq_lens.data_ptr(), q_codes.data_ptr(), sel_idx.data_ptr(), sel_cnt.data_ptr(),
-                                float(sm_scale), out.data_ptr(), workspace.data_ptr(),
-                                workspace.numel() * workspace.element_size(), status.data_ptr(),
-                                torch.cuda.current_stream(q.device).cuda_stream)
+                                float(sm_scale), out.data_ptr(), workspace.data_ptr(), have, status.data_ptr(),
+                                torch.cuda.current_stream(device).cuda_stream)
     if rc != _lib.HA_OK:
         raise RuntimeError(f"ha_decode_step failed: {_lib.status_str(rc)} (status {rc})")
+    # what was written counts as modified in place for autograd's saved tensors (inference tensors carry no version)
+    torch.autograd.graph.increment_version([t for t in (k_pages, v_pages, hash_pages, q_codes, sel_idx, sel_cnt, workspace,
+                                                        status, out) if not t.is_inference()])
 
 
-@decode_step.register_fake
+
+
 def _decode_step_fake(q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk,
                       q_codes, sel_idx, sel_cnt, workspace, status, out,
                       init_budget, recent_budget, heavy_budget, sm_scale, eval_mode=0, retrieve_depth=0,
                       num_hash_layers=3) -> None:
     return None
+
+
+_LIB.impl("decode_step", _decode_step_cuda, "CUDA")
+_LIB.impl("decode_step", _autograd, "AutogradCUDA", with_keyset=True)
+torch.library.register_fake("hashattn::decode_step", _decode_step_fake, lib=_LIB)
 
 
 def decode_step_op(ctx, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,

@@ -826,6 +826,32 @@ def test_registered_torch_operator_gives_the_library_result_eagerly_and_in_a_gra
 
 
 @pytest.mark.gpu
+def test_registered_operator_below_autograd(device):
+    """The operator has no backward: inputs that require grad leave its results unconnected, what it writes counts as
+    modified in place, function transforms are refused, and inference mode works."""
+    usa = synthetic.make_usa(4, 128, 6, True)
+    inp = synthetic.make_decode_inputs(109, [300], 4, 1)
+    cache, ctx = build(device, inp.q, inp.k, inp.v, ha.Budget(16, 1.0 / 8, 16), usa)
+    ctx.hash_prefill()
+    q, k, v = inp.q.to(device, torch.bfloat16), cache.read_kv(0)[0][None, :, -1], cache.read_kv(0)[1][None, :, -1]
+    k, v = k.to(torch.bfloat16).contiguous(), v.to(torch.bfloat16).contiguous()
+    want = ctx.decode_step(q, k, v)
+    out = torch.zeros_like(q)
+    version = out._version
+    ha.decode_step_op(ctx, q.clone().requires_grad_(), k, v, out=out)
+    assert torch.equal(out, want) and not out.requires_grad and out._version > version
+    x = torch.ones_like(q, dtype=torch.float32).requires_grad_()
+    y = (x * out).sum()  # saves `out`
+    ha.decode_step_op(ctx, q, k, v, out=out)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: ha.decode_step_op(ctx, t, k, v).float().sum())(q)
+    with torch.inference_mode():
+        assert torch.equal(ha.decode_step_op(ctx, q, k, v), want)
+    ctx.check_status()
+
+
 def test_cuda_graph_replay(device):
     usa = synthetic.make_usa(8, 128, 0, True)
     inp = synthetic.make_decode_inputs(100, [2000], 8, 2)
