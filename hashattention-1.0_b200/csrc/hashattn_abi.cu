@@ -297,7 +297,7 @@ bool use_cluster_select(const ha_shape_t* shape) {
     const long long max_tokens = (long long)shape->max_pages * kPage;
     const long long units = (long long)shape->batch * shape->num_kv_heads;
     const int forced = option(HA_OPT_CLUSTER_SELECT);  // 0 never, 1 whenever the sequences fit the kernel
-    if (forced == 0 || max_tokens > 2LL * kClRoundTokens) return false;
+    if (forced == 0 || max_tokens > kClMaxTokens) return false;
     return forced == 1 || units <= 8;
 }
 
@@ -835,11 +835,10 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     const long long max_tokens = (long long)shape->max_pages * kPage;
     if (!plan_only && use_cluster_select(shape)) {
         const dim3 cgrid(kClCtas, shape->num_kv_heads, shape->batch);
-        const cudaError_t e = max_tokens <= kCsMaxTokens
-            ? launch(score_select_short_kernel, cgrid, dim3(kCsThreads), s, kClCtas, p)
-            : max_tokens <= kClRoundTokens
-            ? launch(score_select_cluster_kernel<1>, cgrid, dim3(kClThreads), s, kClCtas, p)
-            : launch(score_select_cluster_kernel<2>, cgrid, dim3(kClThreads), s, kClCtas, p);
+        const cudaError_t e =
+            max_tokens <= cluster_tokens(512, 1)  ? launch(score_select_cluster_kernel<512, 1>, cgrid, dim3(512), s, kClCtas, p)
+            : max_tokens <= cluster_tokens(1024, 1) ? launch(score_select_cluster_kernel<1024, 1>, cgrid, dim3(1024), s, kClCtas, p)
+                                                    : launch(score_select_cluster_kernel<1024, 2>, cgrid, dim3(1024), s, kClCtas, p);
         return e == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
     }
     if (launch_score_hist(shape, g.chunk_pages, p, shape->num_kv_heads, s) != cudaSuccess) return HA_ERR_LAUNCH;

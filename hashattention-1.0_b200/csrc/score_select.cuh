@@ -473,306 +473,33 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
 }
 
 // ------------------------------------------------------------------------------------------
-// Single-kernel variant for short sequences (up to ROUNDS * 32768 tokens): one cluster of 8 CTAs
-// x 1024 threads owns one (sequence, kv-head). A CTA scores 4096 tokens per round (4 per lane),
-// keeps the packed scores in registers, and the 8 CTAs exchange their 4 x 33 histograms through
-// distributed shared memory instead of global memory - so the hash pages are read once, there
-// is no second pass, no histogram traffic and no kernel hand-over between scoring and
-// selection. Token order is (round, CTA rank, warp, it, lane); results are identical to
-// score_hist_kernel + select_kernel.
+// Single-kernel variant for few units of up to 65536 tokens, where the chain of dependent steps is all there is (hash
+// words, exchange, threshold, counts, emission): a cluster of 8 CTAs owns one (sequence, kv-head), CTA r the r-th eighth
+// of the sequence, a warp one block of 128 consecutive tokens, held in registers (two blocks, 32 apart, beyond 32768
+// tokens). A CTA so has one histogram and one place in each list. The CTAs push their histograms into one another's shared
+// memory (a remote store costs the sender nothing, a remote read a round trip), the threshold warps add them up on the
+// way, and the counts of the blocks are scanned by one warp per head. The hash pages are read once, and no histogram, plan
+// or score byte passes through global memory. Results are identical to score_hist_kernel + select_attend_kernel.
+//
+// Threads follow the length, so that a warp has one block where 1024 threads allow it: with 512 threads (which several
+// CTAs on an SM and the neighbouring kernels can live with) up to 16384 tokens. Decode step of one sequence x 8 kv-heads,
+// against CTAs that walked the sequence in common rounds of 32768 tokens: 13.6 -> 11.6 us at 700 tokens, 19.1 -> 15.1 at
+// 4096 (1/4 budget), 16.3 -> 13.7 at 16000, 15.8 -> 14.4
+// at 20000, 17.8 -> 17.4 at 32768, 30.0 -> 28.0 at 65000.
 // ------------------------------------------------------------------------------------------
-constexpr int kClThreads = 1024;
-constexpr int kClWarps = kClThreads / 32;                     // 32 = slots per CTA and round
 constexpr int kClCtas = 8;                                    // portable cluster size
-constexpr int kClCtaTokens = kClThreads * kLaneTokens;        // 4096 tokens per CTA and round
-constexpr int kClRoundTokens = kClCtas * kClCtaTokens;        // 32768 tokens per cluster and round
-constexpr int kClHistCopies = 8;                              // warp w updates copy w % 8
-
-template <int ROUNDS>
-__global__ void __launch_bounds__(kClThreads, 1) score_select_cluster_kernel(const SelectParams p) {
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int kvh = p.kvh0 + blockIdx.y, b = blockIdx.z;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int Hq = p.Hkv * kGroup;
-    constexpr int kHist = kGroup * kBins;  // 132
-
-    __shared__ uint32_t s_hist[ROUNDS][kClHistCopies][kHist];
-    __shared__ uint32_t s_cta_hist[ROUNDS][kHist];   // read by the other CTAs of the cluster
-    __shared__ int s_tot[kHist];
-    __shared__ int s_bef[ROUNDS][kHist];             // counts in (round, rank) pairs before (rd, this CTA)
-    __shared__ int s_T[kGroup], s_need[kGroup], s_base[ROUNDS][kGroup], s_eqb[ROUNDS][kGroup];
-    __shared__ uint32_t s_sgt[ROUNDS][kClWarps], s_seq[ROUNDS][kClWarps];
-    for (int i = tid; i < ROUNDS * kClHistCopies * kHist; i += kClThreads) (&s_hist[0][0][0])[i] = 0;
-
-    const int S = p.seq_lens[b];
-    const bool s_ok = S >= 1 && S <= p.max_pages * kPage && S <= ROUNDS * kClRoundTokens;
-    const SeqRange r = seq_range(s_ok ? S : 1, p.init_budget, p.recent_budget, p.heavy_budget,
-                                 p.budget_lens != nullptr ? p.budget_lens[b] : -1);
-    auto first_token = [&](int rd) { return rd * kClRoundTokens + rank * kClCtaTokens + warp * (kLaneTokens * 32); };
-    RoundWords rw;
-    const bool active0 = s_ok && first_token(0) < S;  // warp-uniform
-    if (active0) rw.load(p, b, kvh, first_token(0), lane, r);
-
-    pdl_wait();
-    pdl_launch_dependents();
-    if (!s_ok && tid == 0 && rank == 0 && blockIdx.y == 0) report(p.status, HA_ERR_BAD_SEQ_LEN);
-
-    // --- scores of this thread's tokens (packed, byte g = head g) and the CTA's histograms ---------
-    uint32_t sc[ROUNDS][kLaneTokens];
-    int page[ROUNDS];
-    uint32_t cand = 0;  // bit rd * 4 + it
-    bool bad_page = false;
-    const uint4 qn = load_qn(p, b, kvh);
-    __syncthreads();  // s_hist is zero
-#pragma unroll
-    for (int rd = 0; rd < ROUNDS; ++rd) {
-        const int t0 = first_token(rd);
-        const bool act = s_ok && t0 < S;  // warp-uniform
-        page[rd] = 0;
-#pragma unroll
-        for (int it = 0; it < kLaneTokens; ++it) sc[rd][it] = 0;
-        if (!act) continue;
-        if (rd > 0) rw.load(p, b, kvh, t0, lane, r);
-        rw.refresh_newest(p, kvh, t0, lane, r);
-        bad_page |= rw.bad_page;
-        page[rd] = rw.page;
-        cand |= rw.cand << (rd * kLaneTokens);
-        uint32_t* h0 = &s_hist[rd][warp % kClHistCopies][0];
-#pragma unroll
-        for (int it = 0; it < kLaneTokens; ++it) {
-            const uint32_t s0 = __popc(qn.x ^ rw.w[it].x), s1 = __popc(qn.y ^ rw.w[it].y);
-            const uint32_t s2 = __popc(qn.z ^ rw.w[it].z), s3 = __popc(qn.w ^ rw.w[it].w);
-            sc[rd][it] = s0 | (s1 << 8) | (s2 << 16) | (s3 << 24);
-            if (rw.interior || ((rw.cand >> it) & 1u)) {
-                atomicAdd(h0 + s0, 1u);
-                atomicAdd(h0 + kBins + s1, 1u);
-                atomicAdd(h0 + 2 * kBins + s2, 1u);
-                atomicAdd(h0 + 3 * kBins + s3, 1u);
-            }
-            if (p.scores_dbg != nullptr && ((rw.valid >> it) & 1u)) {
-                const size_t pitch = (size_t)p.max_pages * kPage;
-                uint8_t* d = p.scores_dbg + ((size_t)b * Hq + kvh * kGroup) * pitch + t0 + it * 32 + lane;
-                d[0] = (uint8_t)s0;
-                d[pitch] = (uint8_t)s1;
-                d[2 * pitch] = (uint8_t)s2;
-                d[3 * pitch] = (uint8_t)s3;
-            }
-        }
-    }
-    if (bad_page) report(p.status, HA_ERR_BAD_PAGE);
-    __syncthreads();
-    for (int i = tid; i < ROUNDS * kHist; i += kClThreads) {
-        const int rd = i / kHist, bin = i % kHist;
-        uint32_t v = 0;
-#pragma unroll
-        for (int k = 0; k < kClHistCopies; ++k) v += s_hist[rd][k][bin];
-        s_cta_hist[rd][bin] = v;
-    }
-
-    // --- exchange: every CTA sums the histograms of all (round, rank) pairs, and of those before its own
-    cluster.sync();
-    if (tid < kHist) {
-        int tot = 0, run = 0;
-        int bef[ROUNDS];
-#pragma unroll
-        for (int rd = 0; rd < ROUNDS; ++rd) {
-#pragma unroll
-            for (int rk = 0; rk < kClCtas; ++rk) {
-                if (rk == rank) bef[rd] = run;
-                run += (int)*cluster.map_shared_rank(&s_cta_hist[rd][tid], rk);
-            }
-        }
-        tot = run;
-        s_tot[tid] = tot;
-#pragma unroll
-        for (int rd = 0; rd < ROUNDS; ++rd) s_bef[rd][tid] = bef[rd];
-    }
-    __syncthreads();  // s_tot / s_bef complete (the other CTAs may still be reading s_cta_hist)
-
-    // --- threshold, tie quota and output bases per head: warp g scans the 33 bins downwards --------
-    if (warp < kGroup) {
-        const int g = warp;
-        const int n = s_tot[g * kBins + 32 - lane];  // lane l holds bin 32 - l; bin 0 apart
-        int cum = n;
-        // tokens per bin in the (round, rank) pairs before (rd, this CTA); scanned together with the totals
-        // (independent shuffle chains interleave, this section being a serial stretch of the kernel)
-        int nbv[ROUNDS], cumbv[ROUNDS];
-#pragma unroll
-        for (int rd = 0; rd < ROUNDS; ++rd) nbv[rd] = cumbv[rd] = s_bef[rd][g * kBins + 32 - lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, cum, d);
-            int ub[ROUNDS];
-#pragma unroll
-            for (int rd = 0; rd < ROUNDS; ++rd) ub[rd] = __shfl_up_sync(0xffffffffu, cumbv[rd], d);
-            if (lane >= d) {
-                cum += u;
-#pragma unroll
-                for (int rd = 0; rd < ROUNDS; ++rd) cumbv[rd] += ub[rd];
-            }
-        }
-        bool overflow;
-        const Threshold th = pick_threshold(p, n, cum, s_tot[g * kBins], s_ok ? r.hb : 0, overflow);
-        const int T = th.T;
-        if (overflow && lane == 0 && rank == 0) report(p.status, HA_ERR_SEL_OVERFLOW);
-#pragma unroll
-        for (int rd = 0; rd < ROUNDS; ++rd) {
-            const int nb = nbv[rd], cumb = cumbv[rd];
-            const int lt = min(max(32 - T, 0), 31);
-            const int gt_l = __shfl_sync(0xffffffffu, cumb - nb, lt), eq_l = __shfl_sync(0xffffffffu, nb, lt);
-            const int all31 = __shfl_sync(0xffffffffu, cumb, 31);
-            int gt_before = 0, eq_before = 0;
-            if (T >= 1 && T <= 32) {
-                gt_before = gt_l;
-                eq_before = eq_l;
-            } else if (T == 0) {
-                gt_before = all31;
-                eq_before = s_bef[rd][g * kBins];
-            }
-            if (lane == 0) {
-                s_eqb[rd][g] = eq_before;
-                s_base[rd][g] = gt_before + min(eq_before, th.need);
-            }
-        }
-        if (lane == 0) {
-            s_T[g] = T;
-            s_need[g] = th.need;
-            if (rank == 0 && s_ok) p.sel_cnt[(size_t)b * Hq + kvh * kGroup + g] = th.count;
-        }
-    }
-    __syncthreads();
-
-    // --- classify and count per (round, warp) slot -------------------------------------------------
-    const uint32_t t4 = (uint32_t)s_T[0] | ((uint32_t)s_T[1] << 8) | ((uint32_t)s_T[2] << 16) | ((uint32_t)s_T[3] << 24);
-    const uint32_t gt_add = 0x7F7F7F7Fu - t4;
-    auto flags_gt = [&](int rd, int it) {
-        const uint32_t cm = 0u - ((cand >> (rd * kLaneTokens + it)) & 1u);
-        return bytes_gt(sc[rd][it], gt_add) & cm;
-    };
-    auto flags_eq = [&](int rd, int it) {
-        const uint32_t cm = 0u - ((cand >> (rd * kLaneTokens + it)) & 1u);
-        return bytes_eq(sc[rd][it], t4) & cm;
-    };
-#pragma unroll
-    for (int rd = 0; rd < ROUNDS; ++rd) {
-        uint32_t cg_ = 0, ce_ = 0;
-#pragma unroll
-        for (int it = 0; it < kLaneTokens; ++it) {
-            cg_ += flags_gt(rd, it) >> 7;
-            ce_ += flags_eq(rd, it) >> 7;
-        }
-        cg_ = __reduce_add_sync(0xffffffffu, cg_);  // <= 128 per byte: no carry between heads
-        ce_ = __reduce_add_sync(0xffffffffu, ce_);
-        if (lane == 0) {
-            s_sgt[rd][warp] = cg_;
-            s_seq[rd][warp] = ce_;
-        }
-    }
-    __syncthreads();
-
-    // --- per round: prefix over the CTA's 32 warps, then emission as in select_kernel ---------------
-    const uint32_t lt_mask = (1u << lane) - 1u;
-#pragma unroll
-    for (int rd = 0; rd < ROUNDS; ++rd) {
-        // lane = warp index of this round: exclusive prefix sums of the packed counts
-        const uint32_t g4 = s_sgt[rd][lane], e4 = s_seq[rd][lane];
-        const uint32_t g01 = (g4 & 0xffu) | ((g4 & 0xff00u) << 8), g23 = ((g4 >> 16) & 0xffu) | ((g4 >> 24) << 16);
-        const uint32_t e01 = (e4 & 0xffu) | ((e4 & 0xff00u) << 8), e23 = ((e4 >> 16) & 0xffu) | ((e4 >> 24) << 16);
-        uint32_t pg01 = g01, pg23 = g23, pe01 = e01, pe23 = e23;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t a0 = __shfl_up_sync(0xffffffffu, pg01, d), a1 = __shfl_up_sync(0xffffffffu, pg23, d);
-            const uint32_t a2 = __shfl_up_sync(0xffffffffu, pe01, d), a3 = __shfl_up_sync(0xffffffffu, pe23, d);
-            if (lane >= d) {
-                pg01 += a0; pg23 += a1; pe01 += a2; pe23 += a3;
-            }
-        }
-        pg01 -= g01; pg23 -= g23; pe01 -= e01; pe23 -= e23;
-        const uint32_t sg01 = __shfl_sync(0xffffffffu, pg01, warp), sg23 = __shfl_sync(0xffffffffu, pg23, warp);
-        const uint32_t se01 = __shfl_sync(0xffffffffu, pe01, warp), se23 = __shfl_sync(0xffffffffu, pe23, warp);
-        const uint32_t mine_g = s_sgt[rd][warp], mine_e = s_seq[rd][warp];
-        if ((mine_g | mine_e) == 0) continue;  // nothing of any head in this warp's 128 tokens
-        int base_pos[kGroup], eqb[kGroup];
-        uint32_t full4 = 0, straddle = 0;
-#pragma unroll
-        for (int g = 0; g < kGroup; ++g) {
-            const int gt_b = (int)(((g < 2 ? sg01 : sg23) >> ((g & 1) * 16)) & 0xffffu);
-            const int need = s_need[g];
-            eqb[g] = s_eqb[rd][g] + (int)(((g < 2 ? se01 : se23) >> ((g & 1) * 16)) & 0xffffu);
-            const int eq_in = (int)((mine_e >> (8 * g)) & 0xffu);
-            base_pos[g] = s_base[rd][g] + gt_b + (min(eqb[g], need) - min(s_eqb[rd][g], need));
-            if (eqb[g] + eq_in <= need) full4 |= 0x80u << (8 * g);
-            else if (eqb[g] < need) straddle |= 1u << g;
-        }
-        uint32_t selm[kLaneTokens];
-#pragma unroll
-        for (int it = 0; it < kLaneTokens; ++it) selm[it] = flags_gt(rd, it) | (flags_eq(rd, it) & full4);
-        if (straddle != 0) {  // warp-uniform, at most once per (sequence, head): rank ties by token index
-#pragma unroll
-            for (int g = 0; g < kGroup; ++g) {
-                if (!((straddle >> g) & 1u)) continue;
-                int eq_run = eqb[g];
-#pragma unroll
-                for (int it = 0; it < kLaneTokens; ++it) {
-                    const bool eq = (flags_eq(rd, it) >> (8 * g + 7)) & 1u;
-                    const uint32_t m_eq = __ballot_sync(0xffffffffu, eq);
-                    if (eq && eq_run + __popc(m_eq & lt_mask) < s_need[g]) selm[it] |= 0x80u << (8 * g);
-                    eq_run += __popc(m_eq);
-                }
-            }
-        }
-        uint32_t cnt4 = 0, bits = 0;
-#pragma unroll
-        for (int it = 0; it < kLaneTokens; ++it) {
-            cnt4 += selm[it] >> 7;
-            bits |= flags_to_nibble(selm[it]) << (4 * it);
-        }
-        uint32_t excl = cnt4;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, excl, d);
-            if (lane >= d) excl += u;
-        }
-        excl -= cnt4;
-        const int t_lane = first_token(rd) + lane;
-        const int prow0 = page[rd] * kPage + t_lane % kPage;
-        while (bits != 0) {
-            const int i = __ffs(bits) - 1;
-            bits &= bits - 1;
-            const int it = i >> 2, g = i & 3;
-            const int bp = g == 0 ? base_pos[0] : (g == 1 ? base_pos[1] : (g == 2 ? base_pos[2] : base_pos[3]));
-            const int pos = bp + (int)((excl >> (8 * g)) & 0xffu);
-            excl += 1u << (8 * g);
-            if (pos < p.sel_stride) {
-                const size_t o = ((size_t)b * Hq + kvh * kGroup + g) * p.sel_stride + pos;
-                p.sel_idx[o] = t_lane + it * 32;
-                p.sel_rows[o] = prow0 + it * 32;
-            }
-        }
-    }
-    cluster.sync();  // s_cta_hist may be read by the other CTAs until they, too, are past the exchange
-}
-
-// ------------------------------------------------------------------------------------------
-// The same for sequences of up to 16384 tokens, where the chain of dependent steps is all there is (hash words, exchange,
-// threshold, counts, emission): CTA r of the cluster owns the r-th eighth of the sequence, a warp at most 128 consecutive
-// tokens, so that a CTA has one histogram and one place in each list. The CTAs push their histograms into one another's
-// shared memory (a remote store costs the sender nothing, a remote read a round trip), the threshold warps add them up on
-// the way, and the counts of a warp are scanned by one warp per head. Decode step of one sequence x 8 kv-heads: 13.6 ->
-// 11.6 us at 700 tokens, 19.1 -> 15.1 at 4096 (1/4 budget), 16.3 -> 13.7 at 16000. The line is where a warp would own
-// more than one block.
-// ------------------------------------------------------------------------------------------
-constexpr int kCsThreads = 512;
-constexpr int kCsWarps = kCsThreads / 32;
-constexpr int kCsBlock = kLaneTokens * 32;                       // 128 tokens of a warp: half a page
-constexpr int kCsMaxTokens = kClCtas * kCsWarps * kCsBlock;      // 16384
+constexpr int kClBlock = kLaneTokens * 32;                    // 128 tokens of a warp: half a page
+__host__ __device__ constexpr int cluster_tokens(int threads, int blocks) { return kClCtas * (threads / 32) * blocks * kClBlock; }
+constexpr int kClMaxTokens = cluster_tokens(1024, 2);         // 65536
 
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-__global__ void __launch_bounds__(kCsThreads, 1) score_select_short_kernel(const SelectParams p) {
+// kBlocks: blocks of a warp
+template <int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, 1) score_select_cluster_kernel(const SelectParams p) {
+    constexpr int kWarps = kThreads / 32, kSlots = kWarps * kBlocks;  // blocks of a CTA, in token order
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int kvh = p.kvh0 + blockIdx.y, b = blockIdx.z;
@@ -784,20 +511,20 @@ __global__ void __launch_bounds__(kCsThreads, 1) score_select_short_kernel(const
     __shared__ uint32_t s_hist[kCopies][kHist];
     __shared__ uint32_t s_all[kClCtas][kHist];  // every CTA's histogram, pushed by its owner
     __shared__ int s_T[kGroup], s_need[kGroup], s_base[kGroup], s_eqb[kGroup];
-    __shared__ uint2 s_count[kCsWarps];                // per warp: tokens above / at the threshold, a byte per head
-    __shared__ uint32_t s_before[kGroup][kCsWarps];    // exclusive prefix of both, 16 bits each
-    for (int i = tid; i < kCopies * kHist; i += kCsThreads) (&s_hist[0][0])[i] = 0;
+    __shared__ uint2 s_count[kSlots];                // per block: tokens above / at the threshold, a byte per head
+    __shared__ uint32_t s_before[kGroup][kSlots];    // exclusive prefix of both, 16 bits each
+    for (int i = tid; i < kCopies * kHist; i += kThreads) (&s_hist[0][0])[i] = 0;
 
     const int S = p.seq_lens[b];
-    const bool s_ok = S >= 1 && S <= p.max_pages * kPage && S <= kCsMaxTokens;
+    const bool s_ok = S >= 1 && S <= p.max_pages * kPage && S <= cluster_tokens(kThreads, kBlocks);
     const SeqRange r = seq_range(s_ok ? S : 1, p.init_budget, p.recent_budget, p.heavy_budget,
                                  p.budget_lens != nullptr ? p.budget_lens[b] : -1);
     // whole blocks per CTA, spread evenly over the cluster
-    const int nblk = (r.S + kClCtas * kCsBlock - 1) / (kClCtas * kCsBlock);
-    const int t0 = (rank * nblk + warp) * kCsBlock;
-    const bool active = s_ok && warp < nblk && t0 < r.S;  // warp-uniform
+    const int nblk = (r.S + kClCtas * kClBlock - 1) / (kClCtas * kClBlock);
+    auto first_of = [&](int nb) { return (rank * nblk + nb * kWarps + warp) * kClBlock; };
+    auto has = [&](int nb) { return s_ok && nb * kWarps + warp < nblk && first_of(nb) < r.S; };  // warp-uniform
     RoundWords rw;
-    if (active) rw.load(p, b, kvh, t0, lane, r);
+    if (has(0)) rw.load(p, b, kvh, first_of(0), lane, r);
     cluster_arrive_relaxed();  // (the matching wait stands in front of the first push: by then every CTA has started)
 
     pdl_wait();
@@ -806,11 +533,21 @@ __global__ void __launch_bounds__(kCsThreads, 1) score_select_short_kernel(const
 
     const uint4 qn = load_qn(p, b, kvh);
     __syncthreads();  // s_hist is zero
-    uint32_t word[kLaneTokens] = {0u, 0u, 0u, 0u};  // token it * 32 + lane: byte g = head g's score + 1, 0 = not a candidate
-    if (active) {
+    // token it * 32 + lane of a block: byte g = head g's score + 1, 0 = not a candidate
+    uint32_t word[kBlocks][kLaneTokens];
+    int row[kBlocks];  // physical row of the block's first token (used where a token was selected: its page is good)
+    uint32_t* h0 = &s_hist[warp % kCopies][0];
+#pragma unroll
+    for (int nb = 0; nb < kBlocks; ++nb) {
+#pragma unroll
+        for (int it = 0; it < kLaneTokens; ++it) word[nb][it] = 0u;
+        row[nb] = 0;
+        if (!has(nb)) continue;
+        const int t0 = first_of(nb);
+        if (nb > 0) rw.load(p, b, kvh, t0, lane, r);
         rw.refresh_newest(p, kvh, t0, lane, r);
         if (rw.bad_page) report(p.status, HA_ERR_BAD_PAGE);
-        uint32_t* h0 = &s_hist[warp % kCopies][0];
+        row[nb] = rw.page * kPage + t0 % kPage;
 #pragma unroll
         for (int it = 0; it < kLaneTokens; ++it) {
             const uint32_t s0 = __popc(qn.x ^ rw.w[it].x), s1 = __popc(qn.y ^ rw.w[it].y);
@@ -820,7 +557,7 @@ __global__ void __launch_bounds__(kCsThreads, 1) score_select_short_kernel(const
                 atomicAdd(h0 + kBins + s1, 1u);
                 atomicAdd(h0 + 2 * kBins + s2, 1u);
                 atomicAdd(h0 + 3 * kBins + s3, 1u);
-                word[it] = __byte_perm(__byte_perm(s0, s1, 0x1140u), __byte_perm(s2, s3, 0x1140u), 0x5410u) + 0x01010101u;
+                word[nb][it] = __byte_perm(__byte_perm(s0, s1, 0x1140u), __byte_perm(s2, s3, 0x1140u), 0x5410u) + 0x01010101u;
             }
             if (p.scores_dbg != nullptr && ((rw.valid >> it) & 1u)) {
                 const size_t pitch = (size_t)p.max_pages * kPage;
@@ -897,86 +634,103 @@ __global__ void __launch_bounds__(kCsThreads, 1) score_select_short_kernel(const
     // ---- classify: stored bytes are score + 1 (0: no candidate) and are compared with T + 1 >= 1
     const uint32_t t4 = ((uint32_t)s_T[0] | ((uint32_t)s_T[1] << 8) | ((uint32_t)s_T[2] << 16) | ((uint32_t)s_T[3] << 24)) + 0x01010101u;
     const uint32_t gt_add = 0x7F7F7F7Fu - t4, ge_add = 0x80808080u - t4;
-    uint32_t sel[kLaneTokens], eq[kLaneTokens], cgt = 0, ceq = 0;
+    uint32_t cgt[kBlocks], ceq[kBlocks];
 #pragma unroll
-    for (int it = 0; it < kLaneTokens; ++it) {
-        sel[it] = (word[it] + gt_add) & 0x80808080u;
-        eq[it] = (word[it] + ge_add) & 0x80808080u & ~sel[it];
-        cgt += sel[it] >> 7;
-        ceq += eq[it] >> 7;
-    }
-    cgt = __reduce_add_sync(0xffffffffu, cgt);  // <= 128 per byte: no carry between heads
-    ceq = __reduce_add_sync(0xffffffffu, ceq);
-    if (lane == 0) s_count[warp] = make_uint2(cgt, ceq);
-    __syncthreads();
-    if (warp < kGroup) {  // prefix over the CTA's warps: above (low half) and tied (high half)
-        const uint2 c = s_count[lane % kCsWarps];
-        const uint32_t mine = ((c.x >> (8 * warp)) & 0xffu) | (((c.y >> (8 * warp)) & 0xffu) << 16);
-        uint32_t incl = mine;
+    for (int nb = 0; nb < kBlocks; ++nb) {
+        uint32_t cg_ = 0, ce_ = 0;
 #pragma unroll
-        for (int d = 1; d < kCsWarps; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += u;
+        for (int it = 0; it < kLaneTokens; ++it) {
+            const uint32_t gt = (word[nb][it] + gt_add) & 0x80808080u;
+            cg_ += gt >> 7;
+            ce_ += ((word[nb][it] + ge_add) & 0x80808080u & ~gt) >> 7;
         }
-        if (lane < kCsWarps) s_before[warp][lane] = incl - mine;
+        cgt[nb] = __reduce_add_sync(0xffffffffu, cg_);  // <= 128 per byte: no carry between heads
+        ceq[nb] = __reduce_add_sync(0xffffffffu, ce_);
+        if (lane == 0) s_count[nb * kWarps + warp] = make_uint2(cgt[nb], ceq[nb]);
     }
     __syncthreads();
-    if ((cgt | ceq) == 0) return;  // nothing of any head in this warp's tokens
+    if (warp < kGroup) {  // prefix over the CTA's blocks: above (low half) and tied (high half)
+        uint32_t run = 0;
+#pragma unroll
+        for (int k0 = 0; k0 < kSlots; k0 += 32) {
+            const bool in = k0 + lane < kSlots;
+            const uint2 c = s_count[in ? k0 + lane : 0];
+            const uint32_t mine = in ? ((c.x >> (8 * warp)) & 0xffu) | (((c.y >> (8 * warp)) & 0xffu) << 16) : 0u;
+            uint32_t incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += u;
+            }
+            if (in) s_before[warp][k0 + lane] = run + incl - mine;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
 
     // ---- emission: position in the head's list, ties by token index
     const uint32_t lt_mask = (1u << lane) - 1u;
-    int base_pos[kGroup], eqb[kGroup];
-    uint32_t full4 = 0, straddle = 0;
 #pragma unroll
-    for (int g = 0; g < kGroup; ++g) {
-        const uint32_t bf = s_before[g][warp];
-        const int need = s_need[g], eqb0 = s_eqb[g], eq_in = (int)((ceq >> (8 * g)) & 0xffu);
-        eqb[g] = eqb0 + (int)(bf >> 16);
-        base_pos[g] = s_base[g] + (int)(bf & 0xffffu) + (min(eqb[g], need) - min(eqb0, need));
-        if (eqb[g] + eq_in <= need) full4 |= 0x80u << (8 * g);
-        else if (eqb[g] < need) straddle |= 1u << g;
-    }
-#pragma unroll
-    for (int it = 0; it < kLaneTokens; ++it) sel[it] |= eq[it] & full4;
-    if (straddle != 0) {  // warp-uniform, at most once per (sequence, head): rank ties by token index
+    for (int nb = 0; nb < kBlocks; ++nb) {
+        if ((cgt[nb] | ceq[nb]) == 0) continue;  // nothing of any head in this block
+        int base_pos[kGroup], eqb[kGroup];
+        uint32_t full4 = 0, straddle = 0;
 #pragma unroll
         for (int g = 0; g < kGroup; ++g) {
-            if (!((straddle >> g) & 1u)) continue;
-            int eq_run = eqb[g];
+            const uint32_t bf = s_before[g][nb * kWarps + warp];
+            const int need = s_need[g], eqb0 = s_eqb[g], eq_in = (int)((ceq[nb] >> (8 * g)) & 0xffu);
+            eqb[g] = eqb0 + (int)(bf >> 16);
+            base_pos[g] = s_base[g] + (int)(bf & 0xffffu) + (min(eqb[g], need) - min(eqb0, need));
+            if (eqb[g] + eq_in <= need) full4 |= 0x80u << (8 * g);
+            else if (eqb[g] < need) straddle |= 1u << g;
+        }
+        uint32_t sel[kLaneTokens], eq[kLaneTokens];
 #pragma unroll
-            for (int it = 0; it < kLaneTokens; ++it) {
-                const bool e = (eq[it] >> (8 * g + 7)) & 1u;
-                const uint32_t m_eq = __ballot_sync(0xffffffffu, e);
-                if (e && eq_run + __popc(m_eq & lt_mask) < s_need[g]) sel[it] |= 0x80u << (8 * g);
-                eq_run += __popc(m_eq);
+        for (int it = 0; it < kLaneTokens; ++it) {
+            const uint32_t gt = (word[nb][it] + gt_add) & 0x80808080u;
+            eq[it] = (word[nb][it] + ge_add) & 0x80808080u & ~gt;
+            sel[it] = gt | (eq[it] & full4);
+        }
+        if (straddle != 0) {  // warp-uniform, at most once per (sequence, head): rank ties by token index
+#pragma unroll
+            for (int g = 0; g < kGroup; ++g) {
+                if (!((straddle >> g) & 1u)) continue;
+                int eq_run = eqb[g];
+#pragma unroll
+                for (int it = 0; it < kLaneTokens; ++it) {
+                    const bool e = (eq[it] >> (8 * g + 7)) & 1u;
+                    const uint32_t m_eq = __ballot_sync(0xffffffffu, e);
+                    if (e && eq_run + __popc(m_eq & lt_mask) < s_need[g]) sel[it] |= 0x80u << (8 * g);
+                    eq_run += __popc(m_eq);
+                }
             }
         }
-    }
-    uint32_t cnt4 = 0, bits = 0;
+        uint32_t cnt4 = 0, bits = 0;
 #pragma unroll
-    for (int it = 0; it < kLaneTokens; ++it) {
-        cnt4 += sel[it] >> 7;
-        bits |= flags_to_nibble(sel[it]) << (4 * it);
-    }
-    uint32_t excl = cnt4;
+        for (int it = 0; it < kLaneTokens; ++it) {
+            cnt4 += sel[it] >> 7;
+            bits |= flags_to_nibble(sel[it]) << (4 * it);
+        }
+        uint32_t excl = cnt4;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, excl, d);
-        if (lane >= d) excl += u;
-    }
-    excl -= cnt4;
-    const int row_lane = rw.page * kPage + t0 % kPage + lane;
-    while (bits != 0) {
-        const int i = __ffs(bits) - 1;
-        bits &= bits - 1;
-        const int it = i >> 2, g = i & 3;
-        const int bp = g == 0 ? base_pos[0] : (g == 1 ? base_pos[1] : (g == 2 ? base_pos[2] : base_pos[3]));
-        const int pos = bp + (int)((excl >> (8 * g)) & 0xffu);
-        excl += 1u << (8 * g);
-        if (pos < p.sel_stride) {
-            const size_t o = ((size_t)b * Hq + kvh * kGroup + g) * p.sel_stride + pos;
-            p.sel_idx[o] = t0 + lane + it * 32;
-            p.sel_rows[o] = row_lane + it * 32;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, excl, d);
+            if (lane >= d) excl += u;
+        }
+        excl -= cnt4;
+        const int t_lane = first_of(nb) + lane, row_lane = row[nb] + lane;
+        while (bits != 0) {
+            const int i = __ffs(bits) - 1;
+            bits &= bits - 1;
+            const int it = i >> 2, g = i & 3;
+            const int bp = g == 0 ? base_pos[0] : (g == 1 ? base_pos[1] : (g == 2 ? base_pos[2] : base_pos[3]));
+            const int pos = bp + (int)((excl >> (8 * g)) & 0xffu);
+            excl += 1u << (8 * g);
+            if (pos < p.sel_stride) {
+                const size_t o = ((size_t)b * Hq + kvh * kGroup + g) * p.sel_stride + pos;
+                p.sel_idx[o] = t_lane + it * 32;
+                p.sel_rows[o] = row_lane + it * 32;
+            }
         }
     }
 }
