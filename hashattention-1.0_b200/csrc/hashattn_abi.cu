@@ -288,17 +288,31 @@ cudaError_t launch_select_attend(const ha_shape_t* shape, int chunk_pages, const
     return launch(select_attend_merge_kernel, dim3(nheads, shape->batch), dim3(32 * merge_warps(p.nslots)), s, 1, p, chunk_pages * kPage);
 }
 
-// One cluster kernel scores and selects in a single pass when the sequences are short and there are at
-// most 8 (sequence, kv-head) units, one cluster of 8 CTAs x 1024 threads per GPC: at most two rounds each
-// (measured 6.9 us against 9.4 us for the two-pass kernels at B=1, S=32K). With 16 units the clusters no
-// longer run side by side (13.7 us against 11.6 us for the two-pass kernels at B=2), and longer sequences
-// are bandwidth- rather than latency-bound (45 us against 62 us at B=4, S=128K).
+// Selection alone: one cluster kernel scores and selects in a single pass when the sequences are short and there are at
+// most 8 (sequence, kv-head) units, one cluster of 8 CTAs per GPC (measured 6.9 us against 9.4 us for the two-pass kernels
+// at B=1, S=32K). With 16 units the clusters no longer run side by side (13.7 us against 11.6 us at B=2), and longer
+// sequences are bandwidth- rather than latency-bound (45 us against 62 us at B=4, S=128K).
 bool use_cluster_select(const ha_shape_t* shape) {
     const long long max_tokens = (long long)shape->max_pages * kPage;
     const long long units = (long long)shape->batch * shape->num_kv_heads;
     const int forced = option(HA_OPT_CLUSTER_SELECT);  // 0 never, 1 whenever the sequences fit the kernel
     if (forced == 0 || max_tokens > kClMaxTokens) return false;
     return forced == 1 || units <= 8;
+}
+
+// A step: the cluster selection and a gather over its lists, where that gather is short: the cluster variant with few
+// rounds (1 x 8 kv-heads at 32K: 17.5 us against 19.8 with selection and attention in one kernel; 50000 tokens, four
+// rounds: 21.5 / 23.4 with 8 units, 18.5 / 17.8 with 4), or any budget up to 16384 tokens (1 x 8 at 8000 and 1/4: 23.4 /
+// 26.7). Otherwise selection and attention in one kernel gather with more CTAs: 65000 tokens 28.0 / 25.4; 8 x 1 at 33001
+// and 1/8 32.8 / 30.1; under the depth rule, whose lists may hold the whole sequence, 22.2 / 17.2 at 15000 and 28.6 / 19.8
+// at 50000 (4 units).
+bool use_cluster_step(const ha_shape_t* shape, const ha_budget_t* budget) {
+    if (!use_cluster_select(shape)) return false;
+    if (option(HA_OPT_CLUSTER_SELECT) == 1) return true;
+    if (budget->eval_mode == HA_EVAL_SIMPLE && (long long)shape->max_pages * kPage <= cluster_tokens(512, 1)) return true;
+    const AttSplit split = att_split_launch(shape, budget);
+    const long long units = (long long)shape->batch * shape->num_kv_heads;
+    return split.cluster && split.rounds <= (units > 4 ? 4 : 3);
 }
 
 }  // namespace
@@ -927,8 +941,10 @@ static int decode_step_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     int rc = hash_decode_impl(shape, weights, q, k_new, v_new, k_pages, v_pages, hash_pages, page_table,
                               seq_lens, q_codes, nullptr, q_stage, status, stream);
     if (rc != HA_OK) return rc;
+    rc = check_budget(budget);
+    if (rc != HA_OK) return rc;
     const void* q_att = q_stage != nullptr ? q_stage : q;
-    if (!use_cluster_select(shape)) {
+    if (!use_cluster_step(shape, budget)) {
         const bool handover = option(HA_OPT_PLAN_HANDOVER) != 0;
         // scoring + plan, then selection + attention; the merge kernel, last of the step, also leaves the status
         // word in status_out, if given
@@ -980,7 +996,7 @@ int ha_decode_step_rows(const ha_shape_t* shape, const ha_budget_t* budget,
 
 int ha_decode_step_launches(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (check_shape(shape) != HA_OK || check_budget(budget) != HA_OK) return 0;
-    if (use_cluster_select(shape)) {  // encoder, cluster selection, gather (+ merge)
+    if (use_cluster_step(shape, budget)) {  // encoder, cluster selection, gather (+ merge)
         const AttSplit as = att_split_launch(shape, budget);
         return 3 + (as.nsplits > 1 && !as.cluster ? 1 : 0);
     }
@@ -989,7 +1005,7 @@ int ha_decode_step_launches(const ha_shape_t* shape, const ha_budget_t* budget) 
 
 const char* ha_decode_step_path(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (check_shape(shape) != HA_OK || check_budget(budget) != HA_OK) return "invalid";
-    if (use_cluster_select(shape))
+    if (use_cluster_step(shape, budget))
         return att_split_launch(shape, budget).cluster
             ? "hash_decode | score_select_cluster | sparse_gather (cluster)"
             : "hash_decode | score_select_cluster | sparse_gather | sparse_merge";

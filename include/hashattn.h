@@ -127,8 +127,8 @@ const char* ha_status_str(int status);
  * (the one exception, a failure-injection value, is marked).
  *   HA_OPT_CLUSTER_GATHER  -1 library decides, 0 / 1: thread-block-cluster variant of the gather
  *   HA_OPT_CLUSTER_SELECT  -1 library decides (at most 8 (sequence, kv-head) units of at most 65536
- *                          tokens), 0 never, 1 whenever the sequences fit: single-pass cluster kernel
- *                          for scoring + selection
+ *                          tokens; in a step also by the length of the gather that follows), 0 never,
+ *                          1 whenever the sequences fit: single-pass cluster kernel for scoring + selection
  *   HA_OPT_PLAN_HANDOVER   -1 / 1 inside a step the selection kernel takes the plan of each (sequence,
  *                          kv-head) as soon as the scoring kernel has finished it (a ready word per unit in
  *                          the workspace, polled with a bound), 0 it waits for the whole scoring kernel.

@@ -548,6 +548,17 @@ def test_large_batch_in_large_chunks_equals_its_sequences_alone(device, lib_opti
         assert ok, (b, max_abs, rel)
 
 
+@pytest.mark.parametrize("mode,heavy,path", [("simple", 1.0 / 32, "cluster"), ("simple", 1.0 / 8, "select_attend"),
+                                             ("depth", 1.0 / 32, "select_attend")])
+def test_small_step_takes_the_path_its_gather_asks_for(device, mode, heavy, path):
+    """17,000 tokens, 2 units: a short gather follows the cluster selection, a long one (or lists that may hold the whole
+    sequence) runs with selection and attention in one kernel."""
+    usa = synthetic.make_usa(8, 128, 4, True)
+    inp = synthetic.make_decode_inputs(110, [17000], 8, 2)
+    _, _, ctx, _ = run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(64, heavy, 64, mode, 2), shuffle_seed=2)
+    assert path in ctx.step_path()
+
+
 @pytest.mark.parametrize("lens", [[1024, 1025], [127, 128], [2047, 2049], [16384], [16385]])
 def test_cluster_selection_at_the_edges_of_its_parts(device, lens):
     """Sequences around whole blocks of the eight CTAs of a cluster, the largest one the short-sequence kernel takes and
