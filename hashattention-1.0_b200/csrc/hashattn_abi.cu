@@ -160,12 +160,12 @@ Geometry static_geometry(const ha_shape_t* s) {
 }
 
 struct Workspace {
+    uint32_t* arrive;   // [B][Hkv][kArriveStride] arrival counter and histogram totals of the scoring kernel (zero between calls)
     uint32_t* hist;     // [B][Hkv][4*33][nchunks] per-chunk score histograms
     int32_t* sel_rows;  // [B][Hq][sel_stride] physical rows of the selected tokens (single-pass cluster selection)
     float* partials;    // [B][Hq][max(nsplits, nslots)][130] attention partials
     int32_t* plan;      // [B][Hkv][8 + 8 * nchunks] thresholds, tie quotas and per-chunk output bases
     uint8_t* scores;    // [B][Hq][nchunks * chunk tokens] one score byte per token and query head
-    uint32_t* arrive;   // [B][Hkv][kArriveStride] arrival counter and histogram totals of the scoring kernel (zero between calls)
     size_t bytes;
 };
 
@@ -173,12 +173,15 @@ size_t scores_bytes(const ha_shape_t* s, const Geometry& g) {
     return (size_t)s->batch * s->num_kv_heads * kGroup * g.nchunks * g.chunk_pages * kPage;
 }
 
-Workspace carve(const ha_shape_t* s, const ha_budget_t* b, void* base) {
-    const Geometry g = geometry(s, b);
+Workspace carve_cut(const ha_shape_t* s, const ha_budget_t* b, const Geometry& g, void* base) {
     const size_t Hq = (size_t)s->num_kv_heads * kGroup, units = (size_t)s->batch * s->num_kv_heads;
     char* p = static_cast<char*>(base);
     Workspace w;
     size_t off = 0;
+    // The words that have to be zero between calls come first: their place follows from batch and kv-heads alone, so
+    // a caller may change the budgets, the selection rule or sel_stride from one call to the next on one workspace.
+    w.arrive = reinterpret_cast<uint32_t*>(p + off);
+    off += align_up(units * kArriveStride * sizeof(uint32_t));
     w.hist = reinterpret_cast<uint32_t*>(p + off);
     off += align_up(units * g.nchunks * kGroup * kBins * sizeof(uint32_t));
     w.sel_rows = reinterpret_cast<int32_t*>(p + off);
@@ -189,9 +192,16 @@ Workspace carve(const ha_shape_t* s, const ha_budget_t* b, void* base) {
     off += align_up(units * (8 + 8 * (size_t)g.nchunks) * sizeof(int32_t));
     w.scores = reinterpret_cast<uint8_t*>(p + off);
     off += align_up(scores_bytes(s, g));
-    w.arrive = reinterpret_cast<uint32_t*>(p + off);
-    off += align_up(units * kArriveStride * sizeof(uint32_t));
     w.bytes = off;
+    return w;
+}
+
+// The workspace in the cut of these budgets. Its size is that of the largest cut geometry() could choose for the shape, so
+// that it does not depend on the heavy budget or the selection rule.
+Workspace carve(const ha_shape_t* s, const ha_budget_t* b, void* base) {
+    Workspace w = carve_cut(s, b, geometry(s, b), base);
+    for (int cp = 4; cp <= kMaxChunkPages && (cp == 4 || s->max_pages > cp / 2); cp *= 2)
+        w.bytes = std::max(w.bytes, carve_cut(s, b, geometry_of(s, cp), base).bytes);
     return w;
 }
 

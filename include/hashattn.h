@@ -144,7 +144,8 @@ int ha_set_option(int option_key, int value); /* HA_ERR_BAD_ARG for an unknown k
 int ha_get_option(int option_key);
 
 /* Bytes of workspace needed by any entry point below for this shape and these budgets
- * (0 if either is invalid). Host-only arithmetic. */
+ * (0 if either is invalid). Host-only arithmetic. The heavy budget and the selection rule do not change it: one
+ * workspace serves calls of several heavy budgets and of both rules, in any order, without being cleared in between. */
 size_t ha_workspace_bytes(const ha_shape_t* shape, const ha_budget_t* budget);
 
 /* Zeroes the workspace, in particular the arrival counters, histogram totals and ready words of the scoring kernel.

@@ -75,6 +75,19 @@ def test_workspace_bytes():
     assert lib.ha_workspace_bytes(None, bud) == 0
 
 
+@pytest.mark.parametrize("shape_kw", [
+    dict(batch=8, sel_stride=8192), dict(batch=32, max_pages=64, num_pages=2048), dict(batch=4, max_pages=512, num_pages=2048),
+    dict(max_pages=3), dict(batch=16, max_pages=5), dict(batch=16, max_pages=9), dict(batch=2, max_pages=4097, num_kv_heads=1),
+])
+def test_workspace_bytes_do_not_depend_on_the_heavy_budget_or_the_rule(shape_kw):
+    """A caller may change them from call to call on one workspace."""
+    lib = _lib.load()
+    shape = good_shape(**shape_kw)
+    sizes = {lib.ha_workspace_bytes(shape, _lib.HaBudget(128, 128, heavy, mode, 2))
+             for heavy in (0.0, 1.0 / 64, 1.0 / 32, 1.0 / 16, 1.0 / 8, 1.0 / 4, 1.0, 512.0, 1e6) for mode in (0, 1)}
+    assert len(sizes) == 1 and 0 not in sizes
+
+
 @pytest.mark.parametrize("shape_kw,expected", [
     (dict(head_dim=64), _lib.HA_ERR_UNSUPPORTED_DIM),
     (dict(gqa_group=1), _lib.HA_ERR_UNSUPPORTED_DIM),

@@ -548,6 +548,48 @@ def test_large_batch_in_large_chunks_equals_its_sequences_alone(device, lib_opti
         assert ok, (b, max_abs, rel)
 
 
+@pytest.mark.parametrize("batch,Hkv,low,high", [(18, 8, 2049, 9000), (2, 2, 3000, 9000)])
+def test_budgets_and_rules_take_turns_on_one_workspace(device, batch, Hkv, low, high):
+    """One workspace, cleared once, serves steps of several heavy budgets and both selection rules in any order, although
+    they cut the sequences differently (18 sequences x 8 kv-heads: 16-, 8- and 4-page chunks; 2 x 2: the cluster selection
+    and selection + attention in one kernel): every step gives the bits of a step on a workspace of its own."""
+    gen = torch.Generator().manual_seed(batch)
+    lens = [int(x) for x in torch.randint(low, high + 1, (batch,), generator=gen)]
+    cache = ha.PagedHashKVCache(batch, Hkv, max(lens), device, shuffle_seed=7)
+    synthetic.fill_cache_on_device(cache, lens, seed=7)
+    usa = synthetic.make_usa(4 * Hkv, 128, 7, True).packed(device)
+    budgets = [ha.Budget(128, 1.0 / 8, 64), ha.Budget(128, 1.0 / 32, 64), ha.Budget(128, 1.0 / 32, 64, "depth", 2),
+               ha.Budget(128, 1.0 / 16, 64), ha.Budget(128, 1.0 / 4, 64, "depth", 1), ha.Budget(128, 1.0 / 4, 64)]
+    owner = ha.SparseDecodeContext(cache, budgets[2], usa)  # its index buffers cover a whole sequence
+    owner.hash_prefill()
+    gen = torch.Generator(device=device).manual_seed(7)
+    q, k, v = (torch.randn(batch, n, 128, generator=gen, device=device).bfloat16() for n in (4 * Hkv, Hkv, Hkv))
+
+    def context(budget, own_workspace):
+        ctx = copy.copy(owner)
+        ctx.budget, ctx.c_budget = budget, budget.c_struct()
+        ctx.sel_idx, ctx.sel_cnt = torch.zeros_like(owner.sel_idx), torch.zeros_like(owner.sel_cnt)
+        if own_workspace:
+            ctx.workspace = torch.empty_like(owner.workspace)
+            ctx.reset_workspace()
+        return ctx
+
+    want = []
+    for budget in budgets:
+        ctx = context(budget, True)
+        out = ctx.decode_step(q, k, v)
+        ctx.check_status()
+        want.append((out, ctx.sel_cnt, [heavy_from_device(ctx, b, h) for b in (0, batch - 1) for h in range(4 * Hkv)]))
+    for i in (0, 1, 0, 2, 3, 1, 4, 5, 2, 1, 5, 3, 0):
+        ctx = context(budgets[i], False)
+        out = ctx.decode_step(q, k, v)
+        ctx.check_status()
+        assert torch.equal(ctx.sel_cnt, want[i][1]), i
+        got = [heavy_from_device(ctx, b, h) for b in (0, batch - 1) for h in range(4 * Hkv)]
+        assert all(torch.equal(x, y) for x, y in zip(got, want[i][2])), i
+        assert torch.equal(out, want[i][0]), i
+
+
 @pytest.mark.parametrize("mode,heavy,path", [("simple", 1.0 / 32, "cluster"), ("simple", 1.0 / 8, "select_attend"),
                                              ("depth", 1.0 / 32, "select_attend")])
 def test_small_step_takes_the_path_its_gather_asks_for(device, mode, heavy, path):
