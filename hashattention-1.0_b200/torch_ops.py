@@ -18,6 +18,7 @@ from . import _lib
 from .cache import GROUP, HEAD_DIM, PAGE
 from .ops import on_device
 
+_MUTATED = ("k_pages", "v_pages", "hash_pages", "q_codes", "sel_idx", "sel_cnt", "workspace", "status", "out")
 _TENSORS = ("q", "k_new", "v_new", "k_pages", "v_pages", "hash_pages", "page_table", "seq_lens", "wq", "bq", "wk", "bk",
             "q_codes", "sel_idx", "sel_cnt", "workspace", "status", "out")
 
@@ -33,45 +34,18 @@ def _shape_of(q, k_new, k_pages, page_table, sel_idx) -> _lib.HaShape:
                         sel_idx.shape[2])
 
 
-# The operator is defined by its schema and two kernels instead of torch.library.custom_op, whose three Python layers per
-# call (autograd, version counters, backend) took 30 us of host time for these 25 arguments - more than the step takes on
-# the GPU - against 13 us here; what they did is kept: see _autograd and the end of _decode_step_cuda.
-if "_LIB" in globals():  # the module is being reloaded
-    globals()["_LIB"]._destroy()
-_LIB = torch.library.Library("hashattn", "DEF")
-_LIB.define(
-    "decode_step(Tensor q, Tensor k_new, Tensor v_new, Tensor(a3!) k_pages, Tensor(a4!) v_pages, Tensor(a5!) hash_pages, "
-    "Tensor page_table, Tensor seq_lens, Tensor wq, Tensor bq, Tensor wk, Tensor bk, Tensor(a12!) q_codes, "
-    "Tensor(a13!) sel_idx, Tensor(a14!) sel_cnt, Tensor(a15!) workspace, Tensor(a16!) status, Tensor(a17!) out, "
-    "SymInt init_budget, SymInt recent_budget, float heavy_budget, float sm_scale, SymInt eval_mode=0, "
-    "SymInt retrieve_depth=0, SymInt num_hash_layers=3) -> ()", tags=(torch.Tag.pt2_compliant_tag,))
-decode_step = torch.ops.hashattn.decode_step.default
-
-
-class _NoFormula(torch.autograd.Function):
-    """The step below autograd, without a backward: nothing it writes is connected to its inputs, and function transforms
-    (torch.func.grad and the like) are refused, since there is no setup_context."""
-
-    @staticmethod
-    def forward(ctx, *args):
-        with torch._C._AutoDispatchBelowAutograd():
-            return decode_step(*args)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        raise RuntimeError("Trying to backward through hashattn::decode_step but no autograd formula was registered.")
-
-
-def _autograd(keyset, *args):
-    if torch.is_grad_enabled() and any([a.requires_grad for a in args[:len(_TENSORS)]]):
-        return _NoFormula.apply(*args)
-    return decode_step.redispatch(keyset & torch._C._after_autograd_keyset, *args)
-
-
-def _decode_step_cuda(q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk,
-                      q_codes, sel_idx, sel_cnt, workspace, status, out,
-                      init_budget, recent_budget, heavy_budget, sm_scale, eval_mode=0, retrieve_depth=0,
-                      num_hash_layers=3) -> None:
+# torch.library.custom_op takes about 30 us of host time per call for these 25 arguments (18 more than a schema with two
+# kernels of one's own), but it is what lets the package be loaded twice, counts a call as an in-place change of what it
+# writes (fake tensors included) and offers register_vmap / register_autograd / register_kernel.
+@torch.library.custom_op("hashattn::decode_step", mutates_args=_MUTATED, device_types="cuda")
+def decode_step(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
+                k_pages: torch.Tensor, v_pages: torch.Tensor, hash_pages: torch.Tensor,
+                page_table: torch.Tensor, seq_lens: torch.Tensor,
+                wq: torch.Tensor, bq: torch.Tensor, wk: torch.Tensor, bk: torch.Tensor,
+                q_codes: torch.Tensor, sel_idx: torch.Tensor, sel_cnt: torch.Tensor,
+                workspace: torch.Tensor, status: torch.Tensor, out: torch.Tensor,
+                init_budget: int, recent_budget: int, heavy_budget: float, sm_scale: float,
+                eval_mode: int = 0, retrieve_depth: int = 0, num_hash_layers: int = 3) -> None:
     lib = _lib.load()
     device = q.device
     tensors = (q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk, q_codes, sel_idx, sel_cnt,
@@ -103,23 +77,14 @@ def _decode_step_cuda(q, k_new, v_new, k_pages, v_pages, hash_pages, page_table,
                                 torch.cuda.current_stream(device).cuda_stream)
     if rc != _lib.HA_OK:
         raise RuntimeError(f"ha_decode_step failed: {_lib.status_str(rc)} (status {rc})")
-    # what was written counts as modified in place for autograd's saved tensors (inference tensors carry no version)
-    torch.autograd.graph.increment_version([t for t in (k_pages, v_pages, hash_pages, q_codes, sel_idx, sel_cnt, workspace,
-                                                        status, out) if not t.is_inference()])
 
 
-
-
+@decode_step.register_fake
 def _decode_step_fake(q, k_new, v_new, k_pages, v_pages, hash_pages, page_table, seq_lens, wq, bq, wk, bk,
                       q_codes, sel_idx, sel_cnt, workspace, status, out,
                       init_budget, recent_budget, heavy_budget, sm_scale, eval_mode=0, retrieve_depth=0,
                       num_hash_layers=3) -> None:
     return None
-
-
-_LIB.impl("decode_step", _decode_step_cuda, "CUDA")
-_LIB.impl("decode_step", _autograd, "AutogradCUDA", with_keyset=True)
-torch.library.register_fake("hashattn::decode_step", _decode_step_fake, lib=_LIB)
 
 
 def decode_step_op(ctx, q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor,
