@@ -478,14 +478,18 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
 // of the sequence, a warp one block of 128 consecutive tokens, held in registers (two blocks, 32 apart, beyond 32768
 // tokens). A CTA so has one histogram and one place in each list. The CTAs push their histograms into one another's shared
 // memory (a remote store costs the sender nothing, a remote read a round trip), the threshold warps add them up on the
-// way, and the counts of the blocks are scanned by one warp per head. The hash pages are read once, and no histogram, plan
+// way, and every warp sums the counts of the blocks in front of its own. The hash pages are read once, and no histogram, plan
 // or score byte passes through global memory. Results are identical to score_hist_kernel + select_attend_kernel.
 //
 // Threads follow the length, so that a warp has one block where 1024 threads allow it: with 512 threads (which several
 // CTAs on an SM and the neighbouring kernels can live with) up to 16384 tokens. Decode step of one sequence x 8 kv-heads,
-// against CTAs that walked the sequence in common rounds of 32768 tokens: 13.6 -> 11.6 us at 700 tokens, 19.1 -> 15.1 at
-// 4096 (1/4 budget), 16.3 -> 13.7 at 16000, 15.8 -> 14.4
-// at 20000, 17.8 -> 17.4 at 32768, 30.0 -> 28.0 at 65000.
+// against CTAs of 1024 threads that walked the sequence in common rounds of 32768 tokens and read one another's
+// histograms (both in turn, mean over placements of the buffers, +-0.05 us): 13.3 -> 11.3 us at 700 tokens, 20.5 -> 16.1
+// at 4096 (1/4 budget), 17.4 -> 14.2 at 16000, 16.8 -> 15.6 at 20000, 18.2 -> 17.8 at 28000, 22.4 -> 20.2 at 40000, 24.0 ->
+// 22.3 at 50000; at 32768, where the division of the work is the same, 18.15 -> 18.22 on one box and 17.97 -> 17.71 on
+// another. 8 sequences x 1 kv-head at 33001: 20.3 -> 19.0. With the blocks' prefixes scanned by one warp per head behind a
+// barrier of its own, instead of the sums every warp makes for itself: 18.59 and 18.07 at 32768, 20.4 at 8 x 33001, 21.1
+// at 40000, 0.1 to 0.2 us more than now at the others.
 // ------------------------------------------------------------------------------------------
 constexpr int kClCtas = 8;                                    // portable cluster size
 constexpr int kClBlock = kLaneTokens * 32;                    // 128 tokens of a warp: half a page
@@ -512,7 +516,6 @@ __global__ void __launch_bounds__(kThreads, 1) score_select_cluster_kernel(const
     __shared__ uint32_t s_all[kClCtas][kHist];  // every CTA's histogram, pushed by its owner
     __shared__ int s_T[kGroup], s_need[kGroup], s_base[kGroup], s_eqb[kGroup];
     __shared__ uint2 s_count[kSlots];                // per block: tokens above / at the threshold, a byte per head
-    __shared__ uint32_t s_before[kGroup][kSlots];    // exclusive prefix of both, 16 bits each
     for (int i = tid; i < kCopies * kHist; i += kThreads) (&s_hist[0][0])[i] = 0;
 
     const int S = p.seq_lens[b];
@@ -649,38 +652,36 @@ __global__ void __launch_bounds__(kThreads, 1) score_select_cluster_kernel(const
         if (lane == 0) s_count[nb * kWarps + warp] = make_uint2(cgt[nb], ceq[nb]);
     }
     __syncthreads();
-    if (warp < kGroup) {  // prefix over the CTA's blocks: above (low half) and tied (high half)
-        uint32_t run = 0;
-#pragma unroll
-        for (int k0 = 0; k0 < kSlots; k0 += 32) {
-            const bool in = k0 + lane < kSlots;
-            const uint2 c = s_count[in ? k0 + lane : 0];
-            const uint32_t mine = in ? ((c.x >> (8 * warp)) & 0xffu) | (((c.y >> (8 * warp)) & 0xffu) << 16) : 0u;
-            uint32_t incl = mine;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += u;
-            }
-            if (in) s_before[warp][k0 + lane] = run + incl - mine;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-    }
-    __syncthreads();
-
     // ---- emission: position in the head's list, ties by token index
     const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
     for (int nb = 0; nb < kBlocks; ++nb) {
         if ((cgt[nb] | ceq[nb]) == 0) continue;  // nothing of any head in this block
+        // what the CTA's blocks in front of this one hold, 16 bits per head (at most 64 blocks of at most 128). Every warp
+        // adds them up for itself: a scan by one warp per head costs a second barrier of all threads (times above).
+        uint32_t gt01 = 0, gt23 = 0, eq01 = 0, eq23 = 0;
+#pragma unroll
+        for (int k = 0; k <= nb; ++k) {
+            const bool in = lane < kWarps && (k < nb || lane < warp);
+            const uint2 c = in ? s_count[k * kWarps + lane] : make_uint2(0u, 0u);
+            gt01 += __byte_perm(c.x, 0u, 0x4140u);
+            gt23 += __byte_perm(c.x, 0u, 0x4342u);
+            eq01 += __byte_perm(c.y, 0u, 0x4140u);
+            eq23 += __byte_perm(c.y, 0u, 0x4342u);
+        }
+        gt01 = __reduce_add_sync(0xffffffffu, gt01);
+        gt23 = __reduce_add_sync(0xffffffffu, gt23);
+        eq01 = __reduce_add_sync(0xffffffffu, eq01);
+        eq23 = __reduce_add_sync(0xffffffffu, eq23);
         int base_pos[kGroup], eqb[kGroup];
         uint32_t full4 = 0, straddle = 0;
 #pragma unroll
         for (int g = 0; g < kGroup; ++g) {
-            const uint32_t bf = s_before[g][nb * kWarps + warp];
+            const int gt_before = (int)(((g < 2 ? gt01 : gt23) >> (16 * (g & 1))) & 0xffffu);
+            const int eq_before = (int)(((g < 2 ? eq01 : eq23) >> (16 * (g & 1))) & 0xffffu);
             const int need = s_need[g], eqb0 = s_eqb[g], eq_in = (int)((ceq[nb] >> (8 * g)) & 0xffu);
-            eqb[g] = eqb0 + (int)(bf >> 16);
-            base_pos[g] = s_base[g] + (int)(bf & 0xffffu) + (min(eqb[g], need) - min(eqb0, need));
+            eqb[g] = eqb0 + eq_before;
+            base_pos[g] = s_base[g] + gt_before + (min(eqb[g], need) - min(eqb0, need));
             if (eqb[g] + eq_in <= need) full4 |= 0x80u << (8 * g);
             else if (eqb[g] < need) straddle |= 1u << g;
         }

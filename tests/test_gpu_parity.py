@@ -499,12 +499,25 @@ def test_fused_step_replays_bit_identically_from_a_cuda_graph(device, Hkv):
 
 @pytest.mark.parametrize("S", [40000, 70000])
 def test_long_sequence_selection(device, S):
-    """S = 40,000 runs the cluster kernel with two rounds; S = 70,000 the scoring kernel + fused selection /
-    attention. Both against the oracle."""
+    """S = 40,000 runs the cluster kernel with two blocks of tokens per warp; S = 70,000 the scoring kernel + fused
+    selection / attention. Both against the oracle."""
     Hq, Hkv = 8, 2
     usa = synthetic.make_usa(Hq, 128, 4, True)
     inp = synthetic.make_decode_inputs(104, [S], Hq, Hkv)
-    run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 32, 128), shuffle_seed=2)
+    _, _, ctx, _ = run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(128, 1.0 / 32, 128), shuffle_seed=2)
+    assert ("score_select_cluster" if S <= 65536 else "select_attend") in ctx.step_path()
+
+
+@pytest.mark.parametrize("S,heavy,mode", [(32768, 1.0 / 32, "simple"), (32769, 1.0 / 32, "simple"), (65536, 1.0 / 32, "simple"),
+                                          (65535, 1.0 / 4, "simple"), (41001, 1.0 / 64, "depth")])
+def test_cluster_selection_of_long_sequences(device, lib_option, S, heavy, mode):
+    """The cluster kernel with every warp's one block full, with a second block for one warp of a CTA, and with both
+    blocks of every warp full (64 per CTA), where a step of the library's choice may take another path; against the oracle."""
+    lib_option("cluster_select", 1)
+    usa = synthetic.make_usa(4, 128, 4, True)
+    inp = synthetic.make_decode_inputs(111, [S], 4, 1)
+    _, _, ctx, _ = run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(64, heavy, 64, mode, 2), shuffle_seed=2)
+    assert "score_select_cluster" in ctx.step_path()
 
 
 @pytest.mark.parametrize("S", [70000, 80000])
