@@ -94,44 +94,26 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + expf(-x)); }
 
-// Sums of N rows (N = 1, 2, 4 or 8) over the 16 lanes of a half-warp: at every step of the butterfly a lane hands half of
-// its rows to its partner and keeps the other half, so N rows take N - 1 + log2(16 / N) shuffles instead of 4 N and every
-// lane ends up with the sum of one row, row spread_row<N>(sub). Each row is added up in the order of half_warp_sum.
+// Sums of N rows (N = 1 or 4) over the 16 lanes of a half-warp. With four rows a lane hands half of its rows to its partner
+// and keeps the other half in the first two steps of the butterfly, so they take 5 shuffles instead of 16 and every lane
+// ends up with the sum of one row, row spread_row<N>(sub). Each row is added up in the order of half_warp_sum.
 template <int N>
 __device__ __forceinline__ float spread_sum(const float (&s)[N], int sub) {
+    static_assert(N == 1 || N == 4, "one row, or four");
     if constexpr (N == 1) {
         return half_warp_sum(s[0]);
     } else {
-        float r[N / 2];
-        const bool upper = (sub & 8) != 0;
+        const bool upper8 = (sub & 8) != 0, upper4 = (sub & 4) != 0;
+        float r[2];
 #pragma unroll
-        for (int i = 0; i < N / 2; ++i) {
-            const float send = upper ? s[i] : s[i + N / 2], keep = upper ? s[i + N / 2] : s[i];
+        for (int i = 0; i < 2; ++i) {
+            const float send = upper8 ? s[i] : s[i + 2], keep = upper8 ? s[i + 2] : s[i];
             r[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
         }
-        if constexpr (N == 2) {
-            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 4);
-            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 2);
-            r[0] += __shfl_xor_sync(0xffffffffu, r[0], 1);
-            return r[0];
-        } else {
-            float t[N / 4];
-            const bool upper4 = (sub & 4) != 0;
-#pragma unroll
-            for (int i = 0; i < N / 4; ++i) {
-                const float send = upper4 ? r[i] : r[i + N / 4], keep = upper4 ? r[i + N / 4] : r[i];
-                t[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-            }
-            if constexpr (N == 4) {
-                t[0] += __shfl_xor_sync(0xffffffffu, t[0], 2);
-            } else {
-                static_assert(N == 8, "up to 8 rows");
-                const bool upper2 = (sub & 2) != 0;
-                const float send = upper2 ? t[0] : t[1], keep = upper2 ? t[1] : t[0];
-                t[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-            }
-            return t[0] + __shfl_xor_sync(0xffffffffu, t[0], 1);
-        }
+        const float send = upper4 ? r[0] : r[1], keep = upper4 ? r[1] : r[0];
+        float t = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        return t + __shfl_xor_sync(0xffffffffu, t, 1);
     }
 }
 // the row whose sum lane `sub` of a half-warp ends up with; 16 / N lanes hold the same one, the first of them has
@@ -139,20 +121,16 @@ __device__ __forceinline__ float spread_sum(const float (&s)[N], int sub) {
 template <int N>
 __device__ __forceinline__ int spread_row(int sub) { return sub / (16 / N); }
 
-// Thread mapping: kWarps warps; a half-warp (16 lanes x 8 columns) covers one 128-wide weight row.
-// In the two hidden layers a warp owns 128 / kWarps consecutive output rows: load j of a lane belongs to
-// row 2j + (lane >> 4) of them. In the last layer it owns 32 / kWarps rows in the same way.
-constexpr int kMlpWarps = kHashDecodeThreads / 32;   // 16
-template <int kWarps>
-struct MlpRows {
-    static constexpr int kHid = kHidden / kWarps / 2;   // rows per half-warp in a hidden layer
-    static constexpr int kOut = kCodeBits / kWarps / 2;  // ... in the last one
-};
+// Thread mapping: 16 warps; a half-warp (16 lanes x 8 columns) covers one 128-wide weight row.
+// In the two hidden layers a warp owns 8 consecutive output rows: load j of a lane belongs to
+// row 2j + (lane >> 4) of them. In the last layer it owns 2 rows in the same way.
+constexpr int kMlpWarps = kHashDecodeThreads / 32;  // 16
+constexpr int kHid = kHidden / kMlpWarps / 2;       // rows per half-warp in a hidden layer: 4
+constexpr int kOut = kCodeBits / kMlpWarps / 2;     // ... in the last one: 1
 
-// One head's MLP held in the registers of a CTA of kWarps warps.
-template <typename WT, int kWarps = kMlpWarps>
+// One head's MLP held in the registers of a 512-thread CTA.
+template <typename WT>
 struct MlpRegs {
-    static constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
     Row8<WT> w0[kHid], w1[kHid], w2[kOut];
     float b0, b1, b2;  // biases of the rows whose sums this lane ends up with
 
@@ -219,10 +197,9 @@ __device__ __forceinline__ void mlp_store(float v, float* dst, int warp, int lan
 //
 // layers: 3 = all of W0, W1, W2; 2 = W0 then W2 (Linear-SiLU-Linear, hashattention_llama.py:112-120);
 // 1 = W2 alone (:121-127).
-template <typename WT, int kWarps, typename F>
-__device__ __forceinline__ void mlp_eval(const MlpRegs<WT, kWarps>& r, const uint4 raw,
+template <typename WT, typename F>
+__device__ __forceinline__ void mlp_eval(const MlpRegs<WT>& r, const uint4 raw,
                                          MlpSmem& sm, int warp, int lane, F&& between, int layers = 3) {
-    constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
     const int col = (lane & 15) * 8;
     float x[8];
     unpack_x8(raw, x);
@@ -245,10 +222,9 @@ __device__ __forceinline__ void mlp_eval(const MlpRegs<WT, kWarps>& r, const uin
 
 // mlp_eval for two rows at once (`sm[0]`, `sm[1]`): the same weights in registers feed both rows, and the two
 // dependent chains (dot, shuffle reduction, SiLU, barrier) interleave, so the pair costs little more than one row.
-template <typename WT, int kWarps, typename F>
-__device__ __forceinline__ void mlp_eval2(const MlpRegs<WT, kWarps>& r, const uint4 raw_a, const uint4 raw_b,
+template <typename WT, typename F>
+__device__ __forceinline__ void mlp_eval2(const MlpRegs<WT>& r, const uint4 raw_a, const uint4 raw_b,
                                           MlpSmem (&sm)[2], int warp, int lane, F&& between, int layers = 3) {
-    constexpr int kHid = MlpRows<kWarps>::kHid, kOut = MlpRows<kWarps>::kOut;
     const int col = (lane & 15) * 8;
     float xa[8], xb[8];
     unpack_x8(raw_a, xa);

@@ -144,12 +144,6 @@ __device__ __forceinline__ uint4 load_qn(const SelectParams& p, int b, int kvh) 
     return make_uint4(~qc.x, ~qc.y, ~qc.z, ~qc.w);
 }
 
-// Per-byte flags (bit 7 of each byte) for packed scores a (bytes <= 32) against packed thresholds.
-// gt_add = 0x7F7F7F7F - T4: byte sum a + 127 - T carries into bit 7 iff a > T (no carry across bytes).
-__device__ __forceinline__ uint32_t bytes_gt(uint32_t a, uint32_t gt_add) { return (a + gt_add) & 0x80808080u; }
-__device__ __forceinline__ uint32_t bytes_eq(uint32_t a, uint32_t t4) {
-    return ~((a ^ t4) + 0x7F7F7F7Fu) & 0x80808080u;  // (x + 127) has bit 7 iff x != 0
-}
 // bit 7 of byte g -> bit g
 __device__ __forceinline__ uint32_t flags_to_nibble(uint32_t f) { return (((f >> 7) * 0x01020408u) >> 24) & 0xFu; }
 
