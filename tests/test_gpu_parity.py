@@ -827,9 +827,10 @@ def test_repeated_steps_grow_the_cache(device):
 
 
 def test_kv_head_partition_is_bit_identical(device):
-    """Sharding by kv-head (what multi-GPU runs do) changes no bit: each shard, cut with the partition
-    module's own functions and run alone, gives the same codes, sets and output as the unsharded run, and
-    the shards' outputs concatenated in rank order are the unsharded output."""
+    """Sharding by kv-head (what multi-GPU runs do) changes no bit where shard and whole take the same kernels and cut the
+    sequences alike, as here: each shard, cut with the partition module's own functions and run alone, gives the same
+    codes, sets and output as the unsharded run, and the shards' outputs concatenated in rank order are the unsharded
+    output."""
     from hashattention_b200 import partition
     Hq, Hkv, world = 16, 4, 2
     usa = synthetic.make_usa(Hq, 128, 0, True)
@@ -863,6 +864,46 @@ def test_kv_head_partition_is_bit_identical(device):
                 assert torch.equal(heavy_from_device(ctx, b, h), heavy_from_device(ctx_full, b, j0 * 4 + h))
     # rank order == kv-head order: what partition.gather_output concatenates on every rank
     assert torch.equal(torch.cat(outs, dim=1).float().cpu(), out_full)
+
+
+@pytest.mark.parametrize("batch,low,high,world", [(24, 3000, 9000, 4),   # 16-page chunks whole, 4-page ones on a shard
+                                                  (4, 1500, 3000, 8)])   # the cluster selection on a shard only
+def test_kv_head_shards_agree_where_their_kernels_or_chunks_differ(device, batch, low, high, world):
+    """The cut of the sequences and the choice of kernels follow the number of (sequence, kv-head) units a GPU holds, so a
+    shard may add its rows up in another order than the whole: codes and sets are the same, outputs equal to rounding."""
+    from hashattention_b200 import partition
+    Hkv = 8
+    gen = torch.Generator().manual_seed(batch)
+    lens = [int(x) for x in torch.randint(low, high + 1, (batch,), generator=gen)]
+    cache = ha.PagedHashKVCache(batch, Hkv, max(lens), device, shuffle_seed=5)
+    synthetic.fill_cache_on_device(cache, lens, seed=5)
+    usa, budget = synthetic.make_usa(4 * Hkv, 128, 5, True).packed(device), ha.Budget(128, 1.0 / 32, 64)
+    gen = torch.Generator(device=device).manual_seed(5)
+    q, k, v = (torch.randn(batch, n, 128, generator=gen, device=device).bfloat16() for n in (4 * Hkv, Hkv, Hkv))
+
+    def step(cache, usa, q, k, v):
+        ctx = ha.SparseDecodeContext(cache, budget, usa)
+        ctx.hash_prefill()
+        out = ctx.decode_step(q, k, v)
+        ctx.check_status()
+        return ctx, out
+
+    ctx_full, full = step(cache, usa, q, k, v)
+    for shard in (0, world - 1):
+        j0, j1 = partition.kv_head_range(Hkv, world, shard)
+        part = copy.copy(cache)
+        part.num_kv_heads = j1 - j0
+        part.k_pages, part.v_pages = cache.k_pages[:, j0:j1].contiguous(), cache.v_pages[:, j0:j1].contiguous()
+        part.hash_pages = torch.zeros_like(cache.hash_pages[:, j0:j1])
+        ctx, out = step(part, usa.slice_heads(4 * j0, 4 * j1), *partition.shard_step_inputs(q, k, v, world, shard))
+        assert torch.equal(ctx.sel_cnt, ctx_full.sel_cnt[:, 4 * j0:4 * j1])
+        for b in range(batch):
+            assert torch.equal(part.read_codes(b), cache.read_codes(b)[4 * j0:4 * j1])
+        for b in (0, batch // 2, batch - 1):
+            for h in range(4 * (j1 - j0)):
+                assert torch.equal(heavy_from_device(ctx, b, h), heavy_from_device(ctx_full, b, 4 * j0 + h)), (b, h)
+        ok, max_abs, rel = helpers.att_close(out.cpu(), full[:, 4 * j0:4 * j1].cpu())
+        assert ok, (shard, max_abs, rel)
 
 
 @pytest.mark.gpu
