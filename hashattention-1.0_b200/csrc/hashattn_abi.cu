@@ -129,7 +129,7 @@ Geometry geometry_of(const ha_shape_t* s, int chunk_pages) {
 //     outweighs its gather: 32 sequences of 16K at a 1/32 budget take 146.9 us with 4-page chunks (32 rows), 117.7 with
 //     8, 104.6 with 16 (128 rows). Far more, and the rows all resident CTAs have asked L2 for no longer fit it:
 //     4 sequences of 128K at 1/4 take 329 us with 4 pages (256 rows), 412 with 8, 482 with 16; 32 x 16K at 1/8: 215 / 216
-//     / 282. In between nothing changes by more than 2 % (32 x 16K - 64K at 1/16: 345 us with 8 pages, 359 with 16).
+//     / 282. In between nothing changes by more than 4 % (32 x 16K - 64K at 1/16: 345 us with 8 pages, 359 with 16).
 //   * at least two waves of CTAs (7 per SM), or the last wave and the uneven lists show: 8 x 16K at 1/32 takes 40.1 us
 //     with 16 pages (1536 CTAs), 38.5 with 8 (2560); 4 x 24K at 1/16 58.7 with 16, 50.5 with 8, 50.0 with 4. A sequence
 //     is not cut into more than 64 chunks for this, and a chunk is not larger than the longest sequence.
@@ -299,9 +299,11 @@ cudaError_t launch_select_attend(const ha_shape_t* shape, int chunk_pages, const
 }
 
 // Selection alone: one cluster kernel scores and selects in a single pass when the sequences are short and there are at
-// most 8 (sequence, kv-head) units, one cluster of 8 CTAs per GPC (measured 6.9 us against 9.4 us for the two-pass kernels
-// at B=1, S=32K). With 16 units the clusters no longer run side by side (13.7 us against 11.6 us at B=2), and longer
-// sequences are bandwidth- rather than latency-bound (45 us against 62 us at B=4, S=128K).
+// most 8 (sequence, kv-head) units. Cluster kernel / two-pass kernels, us: 8 units 3.6 / 6.9 at 4096 tokens, 4.1 / 7.3 at
+// 16384, 5.5 / 8.4 at 32768, 8.7 / 11.0 at 65536; 16 units 4.1 / 7.0, 5.0 / 8.1, 10.4 / 10.9 and 16.7 / 13.4: clusters of
+// 1024 threads then no longer run side by side. Those of 512 threads do (32 units 4.3 / 7.4 at 4096, 5.8 / 10.7 at 16384),
+// but the limit is one for all lengths because a step gains nothing there: 16 units 17.4 / 16.6 at 4096 and 21.7 / 19.3 at
+// 16384, 32 units 28.9 / 18.6 at 4096 (24 units at 16384, alone of those measured, 22.2 / 23.3).
 bool use_cluster_select(const ha_shape_t* shape) {
     const long long max_tokens = (long long)shape->max_pages * kPage;
     const long long units = (long long)shape->batch * shape->num_kv_heads;
@@ -310,12 +312,18 @@ bool use_cluster_select(const ha_shape_t* shape) {
     return forced == 1 || units <= 8;
 }
 
-// A step: the cluster selection and a gather over its lists, where that gather is short: the cluster variant with few
-// rounds (1 x 8 kv-heads at 32K: 17.5 us against 19.8 with selection and attention in one kernel; 50000 tokens, four
-// rounds: 21.5 / 23.4 with 8 units, 18.5 / 17.8 with 4), or any budget up to 16384 tokens (1 x 8 at 8000 and 1/4: 23.4 /
-// 26.7). Otherwise selection and attention in one kernel gather with more CTAs: 65000 tokens 28.0 / 25.4; 8 x 1 at 33001
-// and 1/8 32.8 / 30.1; under the depth rule, whose lists may hold the whole sequence, 22.2 / 17.2 at 15000 and 28.6 / 19.8
-// at 50000 (4 units).
+// A step: the cluster selection and a gather over its lists, where that gather is short; selection and attention in one
+// kernel, which gather with more CTAs, elsewhere. Cluster / one kernel, us for one sequence:
+//   * few rounds of the cluster gather: 32768 tokens at 1/32 15.5 / 16.9 with 4 units, 12.8 / 13.5 with 1; 50000 tokens
+//     (four rounds) 21.7 / 22.8 with 8 units, 19.3 / 18.7 with 4; more rounds: 65000 tokens 26.7 / 24.5; 8 sequences x 1
+//     kv-head at 33001 and 1/8 31.6 / 29.3.
+//   * any budget up to 16384 tokens: at 1/4 23.3 / 26.0 with 8 units of 8000 tokens, of 16384 tokens 29.9 / 30.7 with 8,
+//     24.9 / 26.7 with 4, 21.1 / 24.8 with 2, 17.3 / 22.7 with 1; at 1/8 16.3 / 19.9 with 2, 14.4 / 16.2 with 1.
+//   * not under the depth rule, whose lists may hold the whole sequence: 19.3 / 16.5 at 15000, 29.0 / 19.7 at 50000 (4
+//     units).
+// Rounds follow from sel_stride, the width of the caller's lists, because the gather is cut by it too (att_split_launch):
+// with lists eight times as wide as a 1/32 budget needs, 20.4 / 19.2 at 32768 tokens with 8 units, 18.0 / 17.8 at 20000,
+// 22.1 / 19.2 for 8 x 1 at 33001.
 bool use_cluster_step(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (!use_cluster_select(shape)) return false;
     if (option(HA_OPT_CLUSTER_SELECT) == 1) return true;
