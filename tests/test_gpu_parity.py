@@ -138,6 +138,28 @@ def test_prefill_shapes_match_the_fp32_hash_mlp(device, hkv, lens, first, bf16_w
     assert bool((untouched[~written] == sentinel).all()), "a slot outside [first_token, S) was written"
 
 
+PREFILL_RANGES = [
+    # (kv heads, sequence lengths, first token per sequence or None): more than 32 sequences, ranges that start behind the
+    # 32nd; several short heads per CTA; heads of one tile, fewer and more of them than CTAs; a range that ends in the
+    # first of a head's empty places
+    (4, [129] * 33 + [1] * 5, None),
+    (2, [40] * 70 + [3000], [0] * 70 + [1999]),
+    (16, [300, 128], None),
+    (32, [100], None),
+    (40, [1], None),
+    (8, [1024], None),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bf16_weights", [True, False])
+@pytest.mark.parametrize("hkv,lens,first", PREFILL_RANGES)
+def test_prefill_ranges_cover_every_tile(device, hkv, lens, first, bf16_weights):
+    """The cut of the (head, tile) pairs into ranges of equal cost, at the sizes where it can go wrong: every tile is
+    encoded, with its own head's weights, and nothing else is."""
+    test_prefill_shapes_match_the_fp32_hash_mlp(device, hkv, lens, first, bf16_weights)
+
+
 @pytest.mark.parametrize("bf16_weights", [True, False])
 def test_decode_encoder_matches_oracle(device, bf16_weights):
     """Query codes, appended key codes and the appended K / V rows, bf16 and fp32 weights, batch 5."""
