@@ -161,6 +161,7 @@ Geometry static_geometry(const ha_shape_t* s) {
 
 struct Workspace {
     uint32_t* arrive;   // [B][Hkv][kArriveStride] arrival counter and histogram totals of the scoring kernel (zero between calls)
+    int32_t* ready;     // [B][Hkv][kReadyStride] ready words of the heads' plans (zero between calls)
     uint32_t* hist;     // [B][Hkv][4*33][nchunks] per-chunk score histograms
     int32_t* sel_rows;  // [B][Hq][sel_stride] physical rows of the selected tokens (single-pass cluster selection)
     float* partials;    // [B][Hq][max(nsplits, nslots)][130] attention partials
@@ -182,6 +183,8 @@ Workspace carve_cut(const ha_shape_t* s, const ha_budget_t* b, const Geometry& g
     // a caller may change the budgets, the selection rule or sel_stride from one call to the next on one workspace.
     w.arrive = reinterpret_cast<uint32_t*>(p + off);
     off += align_up(units * kArriveStride * sizeof(uint32_t));
+    w.ready = reinterpret_cast<int32_t*>(p + off);
+    off += align_up(units * kReadyStride * sizeof(int32_t));
     w.hist = reinterpret_cast<uint32_t*>(p + off);
     off += align_up(units * g.nchunks * kGroup * kBins * sizeof(uint32_t));
     w.sel_rows = reinterpret_cast<int32_t*>(p + off);
@@ -371,7 +374,7 @@ SelectParams select_params(const ha_shape_t* shape, const ha_budget_t* budget, c
     p.heavy_budget = budget->heavy_budget;
     p.eval_mode = budget->eval_mode;
     p.depth = budget->retrieve_depth;
-    p.signal = 0;
+    p.ready = nullptr;
     return p;
 }
 
@@ -859,10 +862,10 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     const Geometry g = geometry(shape, budget);
     SelectParams p = select_params(shape, budget, g, q_codes, hash_pages, page_table, seq_lens, sel_idx, sel_cnt,
                                    scores_dbg, status, w.hist, w.plan, w.scores, w.arrive, w.sel_rows, budget_lens);
-    // handover: the caller launches the selection right behind this call; it then takes each unit's plan as soon as
-    // that unit is ready instead of waiting for the whole scoring grid
+    // handover: the caller launches the selection right behind this call; it then takes each head's plan as soon as
+    // it is ready instead of waiting for the whole scoring grid
     const int ho = option(HA_OPT_PLAN_HANDOVER);  // 0: off; 2: the selection waits for an announcement that is not made
-    p.signal = ((!plan_only || handover) && ho != 0 && ho != 2) ? 1 : 0;
+    if ((!plan_only || handover) && ho != 0 && ho != 2) p.ready = w.ready;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const long long max_tokens = (long long)shape->max_pages * kPage;
     if (!plan_only && use_cluster_select(shape)) {
@@ -878,7 +881,7 @@ static int score_select_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     SelectAttendParams sa = select_attend_params(shape, budget, g, w.plan, w.scores, w.partials, sel_idx, nullptr,
                                                  nullptr, nullptr, page_table, seq_lens, budget_lens, 1.0f,
                                                  nullptr, status, nullptr);
-    if (ho != 0) sa.ready = reinterpret_cast<int32_t*>(w.arrive);
+    if (ho != 0) sa.ready = w.ready;
     return launch_select_attend(shape, g.chunk_pages, sa, shape->num_kv_heads * kGroup, false, s) == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
 }
 
@@ -902,7 +905,7 @@ static int select_attend_impl(const ha_shape_t* shape, const ha_budget_t* budget
     SelectAttendParams sa = select_attend_params(shape, budget, g, w.plan, w.scores, w.partials, sel_idx, q, k_pages,
                                                  v_pages, page_table, seq_lens, budget_lens, sm_scale, out,
                                                  status, status_out);
-    if (handover) sa.ready = reinterpret_cast<int32_t*>(w.arrive);  // (the scoring call in front was told the same)
+    if (handover) sa.ready = w.ready;  // (the scoring call in front was told the same)
     return launch_select_attend(shape, g.chunk_pages, sa, shape->num_kv_heads * kGroup, true, static_cast<cudaStream_t>(stream)) ==
                    cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
 }

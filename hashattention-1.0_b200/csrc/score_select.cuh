@@ -57,7 +57,8 @@ struct SelectParams {
     const int32_t* budget_lens;  // [B] or null: the length the heavy budget is a fraction of, if not seq_lens
     uint32_t* hist;            // workspace: [B][Hkv][4*33][nchunks] per chunk: tokens at or above each score
     uint32_t* arrive;          // workspace: [B][Hkv][kArriveStride] chunks of the unit that have published, the unit's
-                               // histogram totals, and the unit's ready word (all 0 between calls)
+                               // histogram totals (all 0 between calls)
+    int32_t* ready;            // workspace: [B][Hkv][kReadyStride] ready words (0 between calls), or null: nobody waits for them
     int32_t* sel_idx;          // [B][Hq][sel_stride] token indices
     int32_t* sel_rows;         // workspace: [B][Hq][sel_stride] page * 256 + slot of the same tokens
     int32_t* sel_cnt;          // [B][Hq]
@@ -70,7 +71,6 @@ struct SelectParams {
     int init_budget, recent_budget;
     double heavy_budget;
     int eval_mode, depth;      // HA_EVAL_*; usa_retrieve_depth (HA_EVAL_DEPTH only)
-    int signal;                // 1: the selection kernel launched right behind consumes the plan unit by unit (ready word)
 };
 
 // One round of one warp: 128 consecutive tokens of one page, token it*32 + lane for it = 0..3.
@@ -206,76 +206,44 @@ __device__ __forceinline__ uint32_t gather_byte(const uint32_t (&a)[NW], int g) 
     return __byte_perm(__byte_perm(a[0], a[1], sel), __byte_perm(a[2], a[3], sel), 0x5410u);
 }
 
-// The plan of one (sequence, kv-head), worked out by one CTA of 256 threads (the one that published the unit's
-// last histogram). The scoring CTAs have added their histograms up in the unit's totals (33 bins x 4 heads, behind
-// the arrival counter) and stored, per chunk, the counts of tokens at or above every score: warp g picks head g's
-// threshold T and tie quota from the totals, thread (head, chunk) reads what its chunk holds at or above T and
-// above T, and a scan over the chunks gives the number of selected and of tied tokens that precede each chunk.
-// The totals are left at zero for the next call.
-constexpr int kPlanChunks = 64;            // chunks per sweep (sequences of more than 64 chunks take several)
 constexpr int kPlanRows = kGroup * kBins;  // 132 (head, bin) rows
 constexpr int kArriveStride = 136;         // words per unit behind p.arrive: the arrival counter, then the 132 totals
-constexpr int kReadyWord = 133;            // ... and the ready word: > 0 while the unit's plan waits for consumers
+constexpr int kReadyStride = 8;            // words per unit behind p.ready: one per head, > 0 while the head's plan waits for
+                                           // CTAs that will take it
 
-struct PlanSmem {
-    int tot[kPlanRows];
-    int T[kGroup], need[kGroup];
-    int warp_gt[kSelWarps], warp_eq[kSelWarps];
-};
-
-__device__ __forceinline__ void select_plan(const SelectParams& p, int b, int kvh, const SeqRange& r, int nchunks_b,
-                                            PlanSmem& sm, int tid) {
-    const int lane = tid & 31, warp = tid >> 5;
-    const int Hq = p.Hkv * kGroup;
-    const uint32_t* hbase = p.hist + ((size_t)b * p.Hkv + kvh) * kPlanRows * p.nchunks;
-    int32_t* plan = p.plan + ((size_t)b * p.Hkv + kvh) * (8 + 8 * p.nchunks);
-    uint32_t* totals = p.arrive + ((size_t)b * p.Hkv + kvh) * kArriveStride + 1;
-    const int pc_shift = nchunks_b <= 32 ? 5 : 6, pc = 1 << pc_shift;  // chunks per sweep: 32 or 64
-
-    // ---- totals per (head, bin) over all chunks
-    if (tid < kPlanRows) {
-        sm.tot[tid] = (int)__ldcg(totals + tid);
-        totals[tid] = 0u;
-    }
-    __syncthreads();
-
-    // ---- T and the tie quota: warp g for head g, lane l holds bin 32 - l
-    if (warp < kGroup) {
-        const int g = warp;
-        const int n = sm.tot[g * kBins + 32 - lane];
-        int cum = n;
+// The plan of one head of a (sequence, kv-head), worked out by warp g of the CTA that published the unit's last histogram.
+// The scoring CTAs have added their histograms up in the unit's totals (33 bins x 4 heads, behind the arrival counter) and
+// stored, per chunk, the counts of tokens at or above every score: the warp picks the head's threshold T and tie quota from
+// the totals (lane l: bin 32 - l), reads what each chunk holds at or above T and above T (lane = chunk), and a scan gives the
+// number of selected and of tied tokens that precede each chunk. The totals are left at zero for the next call. A head is
+// announced by itself and no warp waits for another one. Against a plan of all four heads by 256 threads, with common
+// staging, three barriers and one announcement per unit, scoring and plan take 54.7 us instead of 63.0 for 32 sequences of
+// 16384 - 65536 tokens x 8 kv-heads, 18.6 instead of 21.4 for 4 x 131072, 5.2 instead of 5.7 for 3 x 9001 - 15000 (steps:
+// 32 x 16000 91.4 / 94.0, 4 x 16000 29.8 / 30.2). Left out altogether, with the sums made by the chunks' CTAs, it saved
+// another 0.5 - 1 us here and cost the attention kernel 8 %.
+__device__ __forceinline__ void select_plan(const SelectParams& p, int b, int kvh, const SeqRange& r, int nchunks_b, int g, int lane) {
+    const size_t u = (size_t)b * p.Hkv + kvh;
+    const uint32_t* hbase = p.hist + (u * kPlanRows + g * kBins) * p.nchunks;
+    int32_t* plan = p.plan + u * (8 + 8 * p.nchunks);
+    uint32_t* unit = p.arrive + u * kArriveStride;
+    uint32_t* totals = unit + 1 + g * kBins;
+    const int n = (int)__ldcg(totals + 32 - lane), tot0 = (int)__ldcg(totals);
+    int cum = n;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, cum, d);
-            if (lane >= d) cum += u;
-        }
-        bool overflow;
-        const Threshold th = pick_threshold(p, n, cum, sm.tot[g * kBins], r.hb, overflow);
-        if (lane == 0) {
-            if (overflow) report(p.status, HA_ERR_SEL_OVERFLOW);
-            sm.T[g] = th.T;
-            sm.need[g] = th.need;
-            plan[g] = th.T;
-            plan[4 + g] = th.need;
-            p.sel_cnt[(size_t)b * Hq + kvh * kGroup + g] = th.count;
-        }
+    for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, cum, d);
+        if (lane >= d) cum += up;
     }
-    __syncthreads();
-
-    // ---- per chunk: tokens above T and tokens at T, then exclusive prefixes over the chunks.
-    //      thread = (head g, chunk cl of the sweep): 4 x pc threads, a head's chunks are pc / 32 warps
-    const int g = (tid >> pc_shift) & (kGroup - 1), cl = tid & (pc - 1);
-    const bool works = tid < kGroup * pc;  // warp-uniform
-    const int T = sm.T[g], need = sm.need[g];
-    const int wpg = pc >> 5;  // warps per head: 1 or 2
+    bool overflow;
+    const Threshold th = pick_threshold(p, n, cum, tot0, r.hb, overflow);
+    const uint32_t* ge_row = hbase + (size_t)min(th.T, kBins - 1) * p.nchunks;  // (T = 33 keeps nothing)
     int gt_carry = 0, eq_carry = 0;
-    for (int c0 = 0; c0 < nchunks_b; c0 += pc) {
-        if (c0 > 0) __syncthreads();  // (warp_gt / warp_eq of the previous sweep have been read)
+    for (int c0 = 0; c0 < nchunks_b; c0 += 32) {
+        const int c = c0 + lane;
         int gt = 0, eq = 0;
-        if (works && c0 + cl < nchunks_b) {
-            const uint32_t* col = hbase + (size_t)(g * kBins) * p.nchunks + c0 + cl;
-            const int ge = T < kBins ? (int)__ldcg(col + (size_t)T * p.nchunks) : 0;  // at or above T
-            gt = T + 1 < kBins ? (int)__ldcg(col + (size_t)(T + 1) * p.nchunks) : 0;
+        if (c < nchunks_b && th.T < kBins) {
+            const int ge = (int)__ldcg(ge_row + c);
+            gt = th.T + 1 < kBins ? (int)__ldcg(ge_row + p.nchunks + c) : 0;
             eq = ge - gt;
         }
         int pg = gt, pe = eq;
@@ -287,25 +255,30 @@ __device__ __forceinline__ void select_plan(const SelectParams& p, int b, int kv
                 pe += u1;
             }
         }
-        if (lane == 31) {
-            sm.warp_gt[warp] = pg;
-            sm.warp_eq[warp] = pe;
+        if (c < nchunks_b) {
+            const int eq_before = eq_carry + pe - eq;
+            plan[8 + 8 * c + g] = gt_carry + pg - gt + min(eq_before, th.need);
+            plan[8 + 8 * c + 4 + g] = eq_before;
         }
-        __syncthreads();
-        if (works) {
-            // with two warps per head the upper one adds the lower one's total
-            const int w0 = g * wpg;
-            const bool upper = wpg == 2 && warp == w0 + 1;
-            const int gt_before = gt_carry + (upper ? sm.warp_gt[w0] : 0) + pg - gt;
-            const int eq_before = eq_carry + (upper ? sm.warp_eq[w0] : 0) + pe - eq;
-            const int cc = c0 + cl;
-            if (cc < nchunks_b) {
-                plan[8 + 8 * cc + g] = gt_before + min(eq_before, need);
-                plan[8 + 8 * cc + 4 + g] = eq_before;
-            }
-            gt_carry += sm.warp_gt[w0] + (wpg == 2 ? sm.warp_gt[w0 + 1] : 0);
-            eq_carry += sm.warp_eq[w0] + (wpg == 2 ? sm.warp_eq[w0 + 1] : 0);
-        }
+        gt_carry += __shfl_sync(0xffffffffu, pg, 31);
+        eq_carry += __shfl_sync(0xffffffffu, pe, 31);
+    }
+    if (lane == 0) {
+        plan[g] = th.T;
+        plan[4 + g] = th.need;
+    }
+    // hand the head over: one count per CTA of select_attend_kernel that will take this plan (a chunk each). Those CTAs run
+    // while other units are still being scored; each takes its count back, so the word is zero again when the step is over.
+    __syncwarp();
+    if (lane == 0 && p.ready != nullptr) {
+        __threadfence();  // the warp's stores (ordered before this lane by the barrier) are visible device-wide
+        atomicAdd(p.ready + u * kReadyStride + g, nchunks_b);
+    }
+    totals[32 - lane] = 0u;
+    if (lane == 0) {
+        totals[0] = 0u;
+        if (overflow) report(p.status, HA_ERR_SEL_OVERFLOW);
+        p.sel_cnt[u * kGroup + g] = th.count;
     }
 }
 
@@ -317,7 +290,6 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
     constexpr int chunk_tokens = ROUNDS * kRoundTokens;
 
     __shared__ uint32_t s_hist[kSelWarps][kGroup * kBins];
-    __shared__ PlanSmem s_plan;  // the plan's staging area (last CTA of the unit only)
     __shared__ int s_last;
     for (int i = tid; i < kSelWarps * kGroup * kBins; i += kSelThreads) (&s_hist[0][0])[i] = 0;
 
@@ -448,22 +420,13 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
         uint32_t* counter = unit;
         const uint32_t before = atomicAdd(counter, 1u);
         s_last = before + 1u == (uint32_t)nchunks_b;
-        if (s_last) *counter = 0u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    select_plan(p, b, kvh, r, nchunks_b, s_plan, tid);
-    // ---- hand the unit over: one count per CTA of select_attend_kernel that will take this plan (a chunk of one
-    //      query head each). Those CTAs run while other units are still being scored; each takes its count back,
-    //      so the word is zero again when the step is over.
-    if (p.signal != 0) {
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            atomicAdd(reinterpret_cast<int*>(unit + kReadyWord), nchunks_b * kGroup);
+        if (s_last) {
+            *counter = 0u;
+            __threadfence();  // what the other CTAs made visible before they counted themselves in is read behind this
         }
     }
+    __syncthreads();
+    if (s_last && warp < kGroup) select_plan(p, b, kvh, r, nchunks_b, warp, lane);
 }
 
 // ------------------------------------------------------------------------------------------

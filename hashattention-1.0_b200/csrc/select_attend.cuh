@@ -16,7 +16,7 @@
 // classifies its 1 - 4 KB of score bytes.
 //
 // Inside a decode step the chunk CTAs do not wait for the whole scoring grid: the CTA that finishes the
-// plan of a (sequence, kv-head) announces it in a ready word, a chunk CTA of that unit polls the word
+// plan of a (sequence, kv-head) announces it in a ready word per head, a chunk CTA of that head polls the word
 // (bounded) and goes on, while other units are still being scored. Rows are asked for in L2 as soon as
 // they are known to be attended, so that only the first round of a gather waits for DRAM.
 //
@@ -40,7 +40,7 @@ constexpr int kSaWorkers = kSaThreads / kSaLanes;    // 16 rows are worked on si
 constexpr int kSaRows = 2;                           // rows a worker keeps in flight per round
 constexpr int kSaRoundRows = kSaWorkers * kSaRows;   // 32
 constexpr int kSaWarps = kSaThreads / 32;
-constexpr int kSaReadyPolls = 1 << 20;               // polls of a unit's ready word (200 ns apart) before a CTA gives up
+constexpr int kSaReadyPolls = 1 << 20;               // polls of a head's ready word (200 ns apart) before a CTA gives up
 constexpr int kSaEdgeSlots = 2;  // CTA 0 of a head attends the sink tokens, CTA 1 the recent ones, CTA 2 + c chunk c
 
 // bf16 operands of the mixed-precision multiply-add are taken as they are stored (exact products, fp32
@@ -69,7 +69,7 @@ struct SelectAttendParams {
     float* partials;              // workspace: [B][Hq][nslots][130]
     int32_t* status;
     int32_t* status_out;          // see SparseDecodeParams
-    int32_t* ready;               // the scoring kernel's per-unit words (stride kArriveStride; word kReadyWord is used), or
+    int32_t* ready;               // [B][Hkv][kReadyStride] ready words of the heads' plans, or
                                   // null: the plan and the score bytes are complete when the kernel in front has ended
     int B, Hkv, max_pages, num_pages, sel_stride, nchunks, nslots;
     int h0;                       // first query head of this launch
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kSaThreads, kMinCtas) select_attend_kernel(con
         // The scoring kernel in front is still running, but all of its CTAs have started (it lets its dependents go
         // only then), so the unit's plan arrives without any help from this grid. The wait is bounded all the same.
         if (tid == 0) {
-            int* word = p.ready + ((size_t)b * p.Hkv + kvh) * kArriveStride + kReadyWord;
+            int* word = p.ready + ((size_t)b * p.Hkv + kvh) * kReadyStride + g;
             int v, polls = 0;
             for (;;) {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");

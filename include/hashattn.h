@@ -130,7 +130,7 @@ const char* ha_status_str(int status);
  *                          tokens; in a step also by the length of the gather that follows), 0 never,
  *                          1 whenever the sequences fit: single-pass cluster kernel for scoring + selection
  *   HA_OPT_PLAN_HANDOVER   -1 / 1 inside a step the selection kernel takes the plan of each (sequence,
- *                          kv-head) as soon as the scoring kernel has finished it (a ready word per unit in
+ *                          kv-head) as soon as the scoring kernel has finished it (a ready word per head in
  *                          the workspace, polled with a bound), 0 it waits for the whole scoring kernel.
  *                          2 is a failure-injection hook for tests of that bound: the selection waits, the
  *                          scoring kernel does not announce anything, every waiting CTA gives up after its
