@@ -252,9 +252,9 @@ void prefer_carveout(K kernel, int kernel_id, int percent) {
 // Scoring, histograms and the plan (score_hist_kernel) on the kv-heads [p.kvh0, p.kvh0 + nkvh).
 cudaError_t launch_score_hist(const ha_shape_t* shape, int chunk_pages, const SelectParams& p, int nkvh, cudaStream_t s) {
     const dim3 grid(p.nchunks, nkvh, shape->batch);
-    prefer_carveout(score_hist_kernel<1>, 0, 40);  // 5 CTAs x 13 KB
-    prefer_carveout(score_hist_kernel<2>, 1, 40);
-    prefer_carveout(score_hist_kernel<4>, 2, 40);
+    prefer_carveout(score_hist_kernel<1>, 0, 40);   // 4 CTAs x 8 KB
+    prefer_carveout(score_hist_kernel<2>, 1, 100);  // 6 CTAs x 37 KB
+    prefer_carveout(score_hist_kernel<4>, 2, 100);
     switch (chunk_pages) {
         case 4: return launch(score_hist_kernel<1>, grid, dim3(kSelThreads), s, 1, p);
         case 8: return launch(score_hist_kernel<2>, grid, dim3(kSelThreads), s, 1, p);

@@ -25,11 +25,17 @@
 //
 // Tiling of score_hist_kernel: a CTA of 256 threads owns a chunk of 4 * ROUNDS pages of one (sequence,
 // kv-head) and walks it in rounds of 1024 tokens; in a round warp w owns tokens [128 w, 128 w + 128)
-// (half a page), four per lane. Only four 16-byte loads are in flight per lane, so many CTAs fit on
-// an SM; the loads of a round are issued together without branches between them (indices are
-// clamped into range instead of guarded). Everything that does not depend on the preceding
-// kernel - the sequence length, page ids and the first round's hash words - is fetched before
+// (half a page), four per lane. The words of two rounds are on their way at a time; the copies of a round are issued
+// together without branches between them (indices are clamped into range instead of guarded). Everything that does not
+// depend on the preceding kernel - the sequence length, page ids and the first rounds' hash words - is fetched before
 // the grid-dependency wait.
+//
+// What bounds it: a CTA spends about 1.5 us on its first words and 1.5 us on publishing its counts, so the stream of the
+// others has to cover that. With the words in flight in shared memory (cp.async) six CTAs fit on an SM, where the
+// registers to hold them allowed four: scoring and plan of 32 sequences of 16384 - 65536 tokens x 8 kv-heads take 47.8 us
+// instead of 54.7 (5 CTAs 50.5, 8 47.2), of 4 x 131072 17.7 instead of 18.6 (8 CTAs, with spills: 21.4), of 32 x 20000
+// 21.3 instead of 24.3; the hash words alone would take 28.2, 10.2 and 12.5. Chunks of one round keep them in
+// registers: there the trip through shared memory costs 0.3 us (3 x 9001 - 15000: 5.5 us, else 5.2) and the grid is small.
 //
 // Layout of a score plane: inside every block of 128 tokens the byte of token 32 it + lane (the it-th
 // token of a lane in the warp's round) sits at offset 4 lane + it, so that a lane stores its four
@@ -44,7 +50,7 @@ namespace ha {
 
 namespace cg = cooperative_groups;
 
-constexpr int kShMinCtas = 4;                         // CTAs of score_hist_kernel per SM (64 registers per thread)
+constexpr int kShMinCtas = 6;                         // CTAs of score_hist_kernel<2 or 4> per SM (40 registers per thread, 37 KB)
 constexpr int kRoundPages = 4;                        // pages per round
 constexpr int kRoundTokens = kRoundPages * kPage;     // 1024
 constexpr int kLaneTokens = kRoundTokens / kSelThreads;  // 4 tokens per lane and round
@@ -135,6 +141,31 @@ struct RoundWords {
         for (int it = 0; it < kLaneTokens; ++it)
             if (t0 + it * 32 + lane == r.S - 1 && ((valid >> it) & 1u))
                 w[it] = __ldcg(p.hash_pages + ((size_t)page * p.Hkv + kvh) * kPage + (r.S - 1) % kPage);
+    }
+};
+
+// A round whose words are on their way to shared memory instead of registers: a lane copies its four words (cp.async) and
+// reads back what it has copied itself, so nothing but its own copies has to be waited for. Tokens as in RoundWords.
+struct StagedRound {
+    int page, t0;
+    bool page_ok;
+
+    __device__ __forceinline__ void copy(const SelectParams& p, int kvh, int first, int lane, const SeqRange& r, int pg, uint4* slot) {
+        t0 = first;
+        page_ok = pg >= 0 && pg < p.num_pages;
+        page = page_ok ? pg : 0;
+        const uint4* src = p.hash_pages + ((size_t)page * p.Hkv + kvh) * kPage;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(slot + lane);
+#pragma unroll
+        for (int it = 0; it < kLaneTokens; ++it) {
+            const uint4* w = src + min(t0 + it * 32 + lane, r.S - 1) % kPage;  // clamp: always an in-range slot
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + it * 32 * 16), "l"(w) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    // every token is a candidate, and none is the newest one, whose word the encoder may have written after the copy
+    __device__ __forceinline__ bool interior(const SeqRange& r) const {
+        return page_ok && t0 >= r.lo && t0 + kLaneTokens * 32 <= r.hi && (unsigned)(r.S - 1 - t0) >= (unsigned)(kLaneTokens * 32);
     }
 };
 
@@ -283,15 +314,16 @@ __device__ __forceinline__ void select_plan(const SelectParams& p, int b, int kv
 }
 
 template <int ROUNDS>
-__global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(const SelectParams p) {
+__global__ void __launch_bounds__(kSelThreads, ROUNDS == 1 ? 4 : kShMinCtas) score_hist_kernel(const SelectParams p) {
     const int c = blockIdx.x, kvh = p.kvh0 + blockIdx.y, b = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Hq = p.Hkv * kGroup;
     constexpr int chunk_tokens = ROUNDS * kRoundTokens;
+    constexpr bool kStaged = ROUNDS > 1;  // words in flight to shared memory; else in registers
 
+    __shared__ uint4 s_words[kStaged ? kSelWarps : 1][2][kLaneTokens * 32];
     __shared__ uint32_t s_hist[kSelWarps][kGroup * kBins];
     __shared__ int s_last;
-    for (int i = tid; i < kSelWarps * kGroup * kBins; i += kSelThreads) (&s_hist[0][0])[i] = 0;
 
     const int S = p.seq_lens[b];
     const bool s_ok = S >= 1 && S <= p.max_pages * kPage;
@@ -300,15 +332,22 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
     const SeqRange r = seq_range(s_ok ? S : 1, p.init_budget, p.recent_budget, p.heavy_budget,
                                  p.budget_lens != nullptr ? p.budget_lens[b] : -1);
     // two rounds of hash words are kept in flight: while one is scored the next is on its way
-    RoundWords rw[2];
+    RoundWords rw;
+    StagedRound st[2];
     int pgs[ROUNDS];  // page ids of this warp's half pages, all requested up front
     if (active) {
 #pragma unroll
         for (int rd = 0; rd < ROUNDS; ++rd) pgs[rd] = RoundWords::page_of(p, b, RoundWords::first_token(chunk_start, rd, warp));
-        rw[0].load(p, kvh, RoundWords::first_token(chunk_start, 0, warp), lane, r, pgs[0]);
-        if (ROUNDS > 1 && chunk_start + kRoundTokens < S)
-            rw[1].load(p, kvh, RoundWords::first_token(chunk_start, 1, warp), lane, r, pgs[1]);
+        if constexpr (kStaged) {
+#pragma unroll
+            for (int rd = 0; rd < 2; ++rd)
+                if (chunk_start + rd * kRoundTokens < S)
+                    st[rd].copy(p, kvh, RoundWords::first_token(chunk_start, rd, warp), lane, r, pgs[rd], s_words[warp][rd]);
+        } else {
+            rw.load(p, kvh, RoundWords::first_token(chunk_start, 0, warp), lane, r, pgs[0]);
+        }
     }
+    for (int i = tid; i < kSelWarps * kGroup * kBins; i += kSelThreads) (&s_hist[0][0])[i] = 0;
 
     pdl_wait();
     pdl_launch_dependents();
@@ -328,19 +367,33 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
 #pragma unroll
     for (int rd = 0; rd < ROUNDS; ++rd) {
         if (chunk_start + rd * kRoundTokens >= S) break;
-        RoundWords& cur = rw[rd & 1];
-        const int t0 = RoundWords::first_token(chunk_start, rd, warp);
-        cur.refresh_newest(p, kvh, t0, lane, r);
-        bad_page |= cur.bad_page;
+        StagedRound& cur = st[rd % 2];
+        int t0, page;
+        const uint4* words = s_words[kStaged ? warp : 0][rd % 2] + lane;
+        bool interior, page_ok;
+        if constexpr (kStaged) {
+            if (rd + 1 < ROUNDS && chunk_start + (rd + 1) * kRoundTokens < S) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            t0 = cur.t0;
+            interior = cur.interior(r);
+            page_ok = cur.page_ok;
+            page = cur.page;
+        } else {
+            t0 = RoundWords::first_token(chunk_start, 0, warp);
+            interior = rw.interior;
+            page_ok = pgs[0] >= 0 && pgs[0] < p.num_pages;
+            page = rw.page;
+        }
         uint32_t plane[kGroup] = {0u, 0u, 0u, 0u};  // per head: byte it = score + 1 of this lane's it-th token
-        if (cur.interior && p.scores_dbg == nullptr) {
+        if (interior && p.scores_dbg == nullptr) {
             // the common round: every token is a candidate. The four scores of a token are packed with byte
             // permutes and the 4 x 4 bytes of the lane's tokens transposed at the end.
             uint32_t tok[kLaneTokens];
 #pragma unroll
             for (int it = 0; it < kLaneTokens; ++it) {
-                const uint32_t s0 = __popc(qn.x ^ cur.w[it].x), s1 = __popc(qn.y ^ cur.w[it].y);
-                const uint32_t s2 = __popc(qn.z ^ cur.w[it].z), s3 = __popc(qn.w ^ cur.w[it].w);
+                const uint4 w = kStaged ? words[it * 32] : rw.w[it];
+                const uint32_t s0 = __popc(qn.x ^ w.x), s1 = __popc(qn.y ^ w.y);
+                const uint32_t s2 = __popc(qn.z ^ w.z), s3 = __popc(qn.w ^ w.w);
                 atomicAdd(h0 + s0, 1u);
                 atomicAdd(h0 + kBins + s1, 1u);
                 atomicAdd(h0 + 2 * kBins + s2, 1u);
@@ -353,10 +406,15 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
         } else {
 #pragma unroll
             for (int it = 0; it < kLaneTokens; ++it) {
-                const uint32_t s0 = __popc(qn.x ^ cur.w[it].x), s1 = __popc(qn.y ^ cur.w[it].y);
-                const uint32_t s2 = __popc(qn.z ^ cur.w[it].z), s3 = __popc(qn.w ^ cur.w[it].w);
-                const bool is_cand = cur.interior || ((cur.cand >> it) & 1u);
-                if (is_cand) {
+                const int t = t0 + it * 32 + lane;
+                const bool exists = t < S;
+                bad_page |= exists && !page_ok;
+                uint4 w = kStaged ? words[it * 32] : rw.w[it];
+                if (t == S - 1 && page_ok)  // the newest token's word, which the encoder may have written in the meantime
+                    w = __ldcg(p.hash_pages + ((size_t)page * p.Hkv + kvh) * kPage + t % kPage);
+                const uint32_t s0 = __popc(qn.x ^ w.x), s1 = __popc(qn.y ^ w.y);
+                const uint32_t s2 = __popc(qn.z ^ w.z), s3 = __popc(qn.w ^ w.w);
+                if (page_ok && t >= r.lo && t < r.hi) {
                     atomicAdd(h0 + s0, 1u);
                     atomicAdd(h0 + kBins + s1, 1u);
                     atomicAdd(h0 + 2 * kBins + s2, 1u);
@@ -366,9 +424,9 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
                     plane[2] |= (s2 + 1u) << (8 * it);
                     plane[3] |= (s3 + 1u) << (8 * it);
                 }
-                if (p.scores_dbg != nullptr && ((cur.valid >> it) & 1u)) {
+                if (p.scores_dbg != nullptr && exists && page_ok) {
                     const size_t dpitch = (size_t)p.max_pages * kPage;
-                    uint8_t* d = p.scores_dbg + ((size_t)b * Hq + kvh * kGroup) * dpitch + t0 + it * 32 + lane;
+                    uint8_t* d = p.scores_dbg + ((size_t)b * Hq + kvh * kGroup) * dpitch + t;
                     d[0] = (uint8_t)s0;
                     d[dpitch] = (uint8_t)s1;
                     d[2 * dpitch] = (uint8_t)s2;
@@ -376,9 +434,11 @@ __global__ void __launch_bounds__(kSelThreads, kShMinCtas) score_hist_kernel(con
                 }
             }
         }
-        // the round after next takes this round's registers
-        if (rd + 2 < ROUNDS && chunk_start + (rd + 2) * kRoundTokens < S)
-            cur.load(p, kvh, RoundWords::first_token(chunk_start, rd + 2, warp), lane, r, pgs[rd + 2 < ROUNDS ? rd + 2 : 0]);
+        // the round after next takes this round's place
+        if constexpr (kStaged) {
+            if (rd + 2 < ROUNDS && chunk_start + (rd + 2) * kRoundTokens < S)
+                cur.copy(p, kvh, RoundWords::first_token(chunk_start, rd + 2, warp), lane, r, pgs[rd + 2 < ROUNDS ? rd + 2 : 0], s_words[warp][rd % 2]);
+        }
         // the selection works from these bytes instead of the 16-byte hash words
 #pragma unroll
         for (int g = 0; g < kGroup; ++g)
