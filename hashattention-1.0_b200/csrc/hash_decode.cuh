@@ -445,191 +445,279 @@ hash_decode_kernel(const HashDecodeParams p) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Batched variant for large batches: a CTA evaluates up to 16 sequences of its (head, side) at
-// once as three small GEMMs instead of one sequence after the other. The head's weights are
-// converted to fp32 and stored transposed ([in][out]) in shared memory (144 KB); in a hidden layer
-// warp w owns rows 4 (w % 4) .. +3 and the input slice 32 (w / 4) .. +31, lane l the outputs
-// 4 l .. 4 l + 3: one 16-byte weight load feeds 16 FMAs (4 rows x 4 outputs). The four partial
-// sums of an output are added, biased and passed through SiLU in a second sweep. In the last
-// layer warp = row, lane = output bit, and the warp's ballot is the row's code, so the 16 rows
-// finish (store / append) in parallel. Same arithmetic type (fp32 FMA) as the kernel above; the
-// summation order differs, which only matters inside the |x| < 1e-5 band of the sign.
+// Batched variant: a CTA evaluates 16 sequences of its (head, side) at once, each layer a GEMM of 16 rows on the tensor
+// cores (mma.sync m16n8k16; the 128 rows of a tcgen05 tile would be seven eighths padding). Weights stay in registers in
+// the form in which the matrix instruction takes them: a warp owns one or two n-tiles (8 outputs) of a hidden layer, and in
+// the last layer n-tile w % 4 over a part of the inputs. The order of the inputs inside a product is
+// free, so a lane's share of 32 inputs is 8 consecutive ones: one 16-byte load each of weights and activations feeds two
+// k-steps.
+// Precision: products of two bf16 are exact. An activation is split into three bf16 (24 bits of mantissa), an fp32 weight
+// too, and products below 2^-24 of the largest are left out. The products of the leading parts are summed up by the
+// matrix instruction over 16 inputs only and from there in fp32 additions, so that its truncation stays below theirs.
+// Pre-activations against a 64-bit evaluation, 100 sequences x 32 heads x 2 sides: rms 11e-9 (bf16 weights) and 17e-9
+// (fp32); with fp32 multiply-adds from transposed fp32 weights in shared memory, the form before, 26e-9 and 27e-9.
+// What bounds it: latencies - weights, rows, three GEMMs with a barrier each - at about a third of the issue slots. Against
+// that form, whose multiply-adds from shared memory took 3/4 of its time: 12 - 32 sequences x 8 kv-heads 10.9 -> 4.6 us, 64
+// 18.5 -> 8.0, 100 32.5 -> 14.0; fp32 weights 13.4 -> 8.0 (with parts rounded by cvt instead of truncated 9.5), 21.1 ->
+// 13.6 and 36.0 -> 24.2. With 16 warps for bf16 weights 4.65 and 8.5.
 // ------------------------------------------------------------------------------------------
-constexpr int kHdbRows = 16;   // sequences per CTA and pass
-constexpr int kHdbKSplit = 4;  // input slices of a hidden layer
-// Sequences per CTA from which the batched kernel is used: a pass costs about 8.5 us whatever the number of
-// rows (weights to shared memory + three full GEMM sweeps), the register kernel 3.3 us + 1.5 us per further row.
-constexpr int kHdbMinRows = 6;
-struct HdbSmem {
-    float wt0[kHeadDim][kHidden];    // layer 0, [in][out]
-    float wt1[kHidden][kHidden];     // layer 1
-    float wt2[kHidden][kCodeBits];   // layer 2
-    float bias[kMlpBias];
-    float x[2][kHdbRows][kHidden];   // activations, ping-pong
-    float part[kHdbKSplit][kHdbRows][kHidden];
+constexpr int kHmRows = 16;             // sequences per CTA and pass
+// Warps: each of them reads the 16 rows of activations, so fewer are better (8); fp32 weights, split into parts on the
+// way, want more of them at work and half the registers each.
+template <typename WT> constexpr int kHmWarps = sizeof(WT) == 4 ? 16 : 8;
+constexpr int kHmBlocks = kHidden / 32;             // blocks of 32 inputs: 4
+constexpr int kHmParts = 3;             // bf16 parts of an activation
+constexpr float kHmLargest = 3.3895313892515355e38f;
+constexpr int kHmPitch = kHidden + 32;  // elements: 16-byte reads of two neighbouring rows hit different banks
+// Sequences per CTA from which the batched kernel is used. One encoder with 8 kv-heads (two CTAs per head and side), this
+// kernel / the one above, us: bf16 weights 4.5 / 3.9 with 2 rows per CTA, 4.5 / 5.4 with 3, 4.4 / 6.2 with 4, 4.4 / 7.7 with
+// 5; fp32 weights 8.0 / 7.1 with 4, 8.0 / 8.7 with 5.
+template <typename WT> constexpr int kHmMinRows = sizeof(WT) == 4 ? 5 : 3;
+struct HmSmem {
+    __align__(16) __nv_bfloat16 x[1][kHmRows][kHmPitch];
+    __align__(16) __nv_bfloat16 act[2][kHmParts][kHmRows][kHmPitch];
+    float part[4][kHmRows][kCodeBits];  // sums of the last layer over the warps' parts of the inputs
 };
-constexpr size_t kHdbSmemBytes = sizeof(HdbSmem);
 
+// Eight consecutive weights of one row as bf16 pairs: word(i, s) is part s of the weights 2 i and 2 i + 1
 template <typename WT>
-__device__ __forceinline__ void hdb_load_weights(HdbSmem& sm, const WT* W, const float* bias, int tid) {
-    // A load is 8 consecutive inputs of one output row; consecutive threads take consecutive output
-    // rows of the same input chunk, so a warp's transposed stores hit 32 different banks. All nine
-    // loads of a thread are issued before the first store.
-    constexpr int kPer = kHidden * (kHeadDim / 8) / kHashDecodeThreads;  // 4 loads per thread and hidden layer
-    static_assert(kPer * kHashDecodeThreads == kHidden * (kHeadDim / 8) && kCodeBits * (kHidden / 8) == kHashDecodeThreads,
-                  "thread mapping of the weight transposition");
-    const WT* W1 = W + kHidden * kHeadDim;
-    const WT* W2 = W1 + kHidden * kHidden;
-    Row8<WT> r0[kPer], r1[kPer], r2;
+struct HmWeights;
+template <>
+struct HmWeights<__nv_bfloat16> {
+    static constexpr int kParts = 1;
+    uint4 raw;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { raw = __ldg(reinterpret_cast<const uint4*>(p)); }
+    __device__ __forceinline__ void pin() {}
+    __device__ __forceinline__ void words(int i, uint32_t (&w)[1]) const { w[0] = i == 0 ? raw.x : (i == 1 ? raw.y : (i == 2 ? raw.z : raw.w)); }
+};
+// a and b as three bf16 each, by truncation: 8 bits of the mantissa at a time, 24 in all, so the sum of the parts is exact
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&w)[3]) {
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        const int idx = tid + j * kHashDecodeThreads, o = idx % kHidden, chunk = idx / kHidden;
-        r0[j].load(W + (size_t)o * kHeadDim + chunk * 8);
-        r1[j].load(W1 + (size_t)o * kHidden + chunk * 8);
+    for (int i = 0; i < 3; ++i) {
+        w[i] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);  // the upper halves, a's in the low half
+        a -= bf16_lo(w[i]);
+        b -= bf16_hi(w[i]);
     }
-    r2.load(W2 + (size_t)(tid % kCodeBits) * kHidden + (tid / kCodeBits) * 8);
-    for (int i = tid; i < kMlpBias; i += kHashDecodeThreads) sm.bias[i] = __ldg(bias + i);
-    float e[8];
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        const int idx = tid + j * kHashDecodeThreads, o = idx % kHidden, chunk = idx / kHidden;
-        r0[j].unpack(e);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sm.wt0[chunk * 8 + k][o] = e[k];
-        r1[j].unpack(e);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sm.wt1[chunk * 8 + k][o] = e[k];
+}
+template <>
+struct HmWeights<float> {
+    static constexpr int kParts = 3;
+    float4 a, b;
+    __device__ __forceinline__ void load(const float* p) {
+        a = __ldg(reinterpret_cast<const float4*>(p));
+        b = __ldg(reinterpret_cast<const float4*>(p) + 1);
     }
-    r2.unpack(e);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) sm.wt2[(tid / kCodeBits) * 8 + k][tid % kCodeBits] = e[k];
+    __device__ __forceinline__ void pin() {
+        asm volatile("" : "+f"(a.x), "+f"(a.y), "+f"(a.z), "+f"(a.w), "+f"(b.x), "+f"(b.y), "+f"(b.z), "+f"(b.w));
+    }
+    __device__ __forceinline__ void words(int i, uint32_t (&w)[3]) const {
+        if (i == 0) split3(a.x, a.y, w);
+        else if (i == 1) split3(a.z, a.w, w);
+        else if (i == 2) split3(b.x, b.y, w);
+        else split3(b.z, b.w, w);
+    }
+};
+
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// One hidden layer for 16 rows: partial sums by (row group, input slice), then bias + SiLU.
-__device__ __forceinline__ void hdb_hidden(HdbSmem& sm, const float (*wt)[kHidden], const float* bias, int cur,
-                                           int tid) {
-    const int lane = tid & 31, warp = tid >> 5;
-    const int rg = warp & 3, ks = warp >> 2;
-    float acc[4][4];
+// acc = the 16 rows of A (kA bf16 parts) times TILES n-tiles of weights, over the input blocks [blk0, blk0 + BLOCKS). A lane
+// ends up with rows lane / 4 and lane / 4 + 8, outputs 2 (lane % 4) and the next one, of each tile.
+template <int kA, int TILES, int BLOCKS, typename WT>
+__device__ __forceinline__ void hm_gemm(float (&acc)[TILES][4], const __nv_bfloat16 (*A)[kHmRows][kHmPitch], int blk0,
+                                        const HmWeights<WT> (&w)[TILES][BLOCKS], int lane) {
+    constexpr int kW = HmWeights<WT>::kParts;
+    float small[2][TILES][4];  // products of which one factor is not a leading part, by magnitude
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int n = 0; n < TILES; ++n)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-#pragma unroll 8
-    for (int ii = 0; ii < kHidden / kHdbKSplit; ++ii) {
-        const int i = ks * (kHidden / kHdbKSplit) + ii;
-        const float4 w4 = *reinterpret_cast<const float4*>(&wt[i][lane * 4]);
+        for (int i = 0; i < 4; ++i) acc[n][i] = small[0][n][i] = small[1][n][i] = 0.f;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float xv = sm.x[cur][rg * 4 + r][i];  // broadcast
-            acc[r][0] = fmaf(xv, w4.x, acc[r][0]);
-            acc[r][1] = fmaf(xv, w4.y, acc[r][1]);
-            acc[r][2] = fmaf(xv, w4.z, acc[r][2]);
-            acc[r][3] = fmaf(xv, w4.w, acc[r][3]);
+    for (int k = 0; k < BLOCKS; ++k) {
+        uint4 lo[kA], hi[kA];  // rows lane / 4 and lane / 4 + 8, inputs [8 (lane % 4), + 8) of the block
+#pragma unroll
+        for (int s = 0; s < kA; ++s) {
+            const __nv_bfloat16* src = &A[s][lane / 4][(blk0 + k) * 32 + (lane % 4) * 8];
+            lo[s] = *reinterpret_cast<const uint4*>(src);
+            hi[s] = *reinterpret_cast<const uint4*>(src + 8 * kHmPitch);
+        }
+#pragma unroll
+        for (int n = 0; n < TILES; ++n) {
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+                uint32_t b0[kW], b1[kW];
+                w[n][k].words(2 * kk, b0);
+                w[n][k].words(2 * kk + 1, b1);
+#pragma unroll
+                for (int s = 0; s < kA; ++s) {
+                    const uint32_t a[4] = {kk ? lo[s].z : lo[s].x, kk ? hi[s].z : hi[s].x, kk ? lo[s].w : lo[s].y, kk ? hi[s].w : hi[s].y};
+#pragma unroll
+                    for (int v = 0; v < kW && s + v <= 2; ++v) {
+                        if (s + v == 0) {
+                            float d[4] = {0.f, 0.f, 0.f, 0.f};
+                            mma_16x8x16(d, a, b0[0], b1[0]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) acc[n][i] += d[i];
+                        } else {
+                            mma_16x8x16(small[s + v - 1][n], a, b0[v], b1[v]);
+                        }
+                    }
+                }
+            }
         }
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-        *reinterpret_cast<float4*>(&sm.part[ks][rg * 4 + r][lane * 4]) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-    __syncthreads();
-    {
-        const int row = warp;  // 16 warps, 16 rows; lane l finishes outputs 4 l .. 4 l + 3
-        float4 sum = *reinterpret_cast<const float4*>(&bias[lane * 4]);
+    for (int n = 0; n < TILES; ++n)
 #pragma unroll
-        for (int k = 0; k < kHdbKSplit; ++k) {
-            const float4 p4 = *reinterpret_cast<const float4*>(&sm.part[k][row][lane * 4]);
-            sum.x += p4.x; sum.y += p4.y; sum.z += p4.z; sum.w += p4.w;
+        for (int i = 0; i < 4; ++i) acc[n][i] += small[0][n][i] + small[1][n][i];
+}
+
+// bias + SiLU of a hidden layer's accumulators -> the next layer's input, in three bf16 parts
+template <int TILES>
+__device__ __forceinline__ void hm_activate(__nv_bfloat16 (*dst)[kHmRows][kHmPitch], const float (&acc)[TILES][4],
+                                            const float2 (&bias)[TILES], int warp, int lane) {
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) {
+        const int col = (warp * TILES + n) * 8 + (lane % 4) * 2;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint32_t w[3];
+            // (an infinite activation has no parts: it is held at the largest bf16; a NaN stays one)
+            const float y0 = silu(acc[n][2 * half] + bias[n].x), y1 = silu(acc[n][2 * half + 1] + bias[n].y);
+            split3(y0 > kHmLargest ? kHmLargest : y0, y1 > kHmLargest ? kHmLargest : y1, w);
+#pragma unroll
+            for (int s = 0; s < kHmParts; ++s) *reinterpret_cast<uint32_t*>(&dst[s][lane / 4 + 8 * half][col]) = w[s];
         }
-        *reinterpret_cast<float4*>(&sm.x[cur ^ 1][row][lane * 4]) = make_float4(silu(sum.x), silu(sum.y), silu(sum.z), silu(sum.w));
     }
-    __syncthreads();
 }
 
 template <typename WT>
-__global__ void __launch_bounds__(kHashDecodeThreads, 1)
-hash_decode_batched_kernel(const HashDecodeParams p) {
-    extern __shared__ __align__(16) unsigned char hdb_raw[];
-    HdbSmem& sm = *reinterpret_cast<HdbSmem*>(hdb_raw);
+__global__ void __launch_bounds__(kHmWarps<WT> * 32, 1) hash_decode_batched_kernel(const HashDecodeParams p) {
+    constexpr int kHmTiles = kHidden / (8 * kHmWarps<WT>);  // n-tiles per warp in a hidden layer: 2 or 1
+    constexpr int kSplit = kHmWarps<WT> / 4;                // warps that share an n-tile of the last layer: 2 or 4
+    __shared__ HmSmem sm;
     const int h = blockIdx.x, side = blockIdx.y;
     const int Hq = p.Hkv * kGroup;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int kvh = h / kGroup, g = h % kGroup;
+    const int b_begin = blockIdx.z * p.batch_per_cta;
+    const int b_end = min(p.B, b_begin + p.batch_per_cta);
+    const int half = lane >> 4, sub = lane & 15;  // a half of one of the first eight warps loads and finishes row 2 warp + half
+    auto x_row = [&](int b) {
+        return side == 0 ? p.q + ((size_t)b * Hq + h) * kHeadDim : p.k_new + ((size_t)b * p.Hkv + kvh) * kHeadDim;
+    };
 
-    hdb_load_weights(sm, static_cast<const WT*>(p.w[side]) + (size_t)h * kMlpElems, p.bias[side] + (size_t)h * kMlpBias, tid);
+    // ---- weights and biases: constants, fetched before the dependency wait
+    const WT* W = static_cast<const WT*>(p.w[side]) + (size_t)h * kMlpElems;
+    const float* bias = p.bias[side] + (size_t)h * kMlpBias;
+    HmWeights<WT> w0[kHmTiles][kHmBlocks], w1[kHmTiles][kHmBlocks], w2[1][kHmBlocks / kSplit];
+    float2 b0[kHmTiles], b1[kHmTiles];
+    const int tile2 = warp % 4, blk2 = warp / 4 * (kHmBlocks / kSplit);  // last layer: n-tile and first block of inputs
+#pragma unroll
+    for (int n = 0; n < kHmTiles; ++n) {
+        const int row = (warp * kHmTiles + n) * 8;
+        const WT* src = W + (size_t)(row + lane / 4) * kHidden + (lane % 4) * 8;
+#pragma unroll
+        for (int k = 0; k < kHmBlocks; ++k) {
+            w0[n][k].load(src + k * 32);
+            w1[n][k].load(src + kHidden * kHeadDim + k * 32);
+        }
+        b0[n] = __ldg(reinterpret_cast<const float2*>(bias + row) + lane % 4);
+        b1[n] = __ldg(reinterpret_cast<const float2*>(bias + kHidden + row) + lane % 4);
+    }
+#pragma unroll
+    for (int k = 0; k < kHmBlocks / kSplit; ++k)
+        w2[0][k].load(W + 2 * kHidden * kHidden + (size_t)(tile2 * 8 + lane / 4) * kHidden + (blk2 + k) * 32 + (lane % 4) * 8);
+    const float b2 = __ldg(bias + 2 * kHidden + lane);
+    {
+        // (the rows may still be written by the kernel in front: only their lines are asked for)
+        const int b = b_begin + 2 * warp + half;
+        if (b < b_end && warp < kHmRows / 2 && sub < 2) prefetch_l2(x_row(b) + sub * (kHeadDim / 2));
+    }
 
     pdl_wait();
     pdl_launch_dependents();
 
-    const int b_begin = blockIdx.z * p.batch_per_cta;
-    const int b_end = min(p.B, b_begin + p.batch_per_cta);
-    for (int b0 = b_begin; b0 < b_end; b0 += kHdbRows) {
-        // ---- this warp's row: the sequence's input row (4 elements per lane) and, key side, its append slot
-        const int b = b0 + warp;
-        const bool live = b < b_end;
-        int S = 1, page = 0;
-        // the rows the group's first key head appends (lanes 0-15: K, 16-31: V), requested with the inputs
-        const bool appends = live && side == 1 && g == 0 && p.v_new != nullptr;
-        uint4 app = make_uint4(0u, 0u, 0u, 0u);
-        if (appends) {
-            const size_t src = ((size_t)b * p.Hkv + kvh) * kHeadDim;
-            app = lane < 16 ? *(reinterpret_cast<const uint4*>(p.k_new + src) + lane)
-                            : *(reinterpret_cast<const uint4*>(p.v_new + src) + (lane - 16));
-        }
-        {
-            float4 xv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live) {
-                const __nv_bfloat16* xrow = side == 0 ? p.q + ((size_t)b * Hq + h) * kHeadDim
-                                                      : p.k_new + ((size_t)b * p.Hkv + kvh) * kHeadDim;
-                const uint2 raw = *reinterpret_cast<const uint2*>(xrow + lane * 4);
-                xv = make_float4(bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y));
-                if (side == 0 && p.q_stage != nullptr)
-                    *reinterpret_cast<uint2*>(p.q_stage + ((size_t)b * Hq + h) * kHeadDim + lane * 4) = raw;
-                if (side == 1) {
-                    S = p.seq_lens[b];
-                    page = p.page_table[(size_t)b * p.max_pages + min(max(S - 1, 0) / kPage, p.max_pages - 1)];
-                }
+    for (int r0 = b_begin; r0 < b_end; r0 += kHmRows) {
+        // (the parts of fp32 weights are made anew in every pass: kept, they would take three quarters of the registers)
+#pragma unroll
+        for (int n = 0; n < kHmTiles; ++n)
+#pragma unroll
+            for (int k = 0; k < kHmBlocks; ++k) {
+                w0[n][k].pin();
+                w1[n][k].pin();
             }
-            *reinterpret_cast<float4*>(&sm.x[0][warp][lane * 4]) = xv;
+        // ---- the input rows, 8 elements per lane; key side: the append slot, and the V row the group's first head appends
+        const int row = 2 * warp + half, b = r0 + row;
+        const bool live = row < kHmRows && b < b_end;
+        const bool appends = live && side == 1 && g == 0 && p.v_new != nullptr;
+        uint4 raw = make_uint4(0u, 0u, 0u, 0u), v_raw = raw;
+        int S = 1, page = 0;
+        if (live) {
+            raw = *(reinterpret_cast<const uint4*>(x_row(b)) + sub);
+            if (appends) v_raw = *(reinterpret_cast<const uint4*>(p.v_new + ((size_t)b * p.Hkv + kvh) * kHeadDim) + sub);
+            if (side == 1) {
+                S = p.seq_lens[b];
+                page = p.page_table[(size_t)b * p.max_pages + min(max(S - 1, 0) / kPage, p.max_pages - 1)];
+            }
+            if (side == 0 && p.q_stage != nullptr) *(reinterpret_cast<uint4*>(p.q_stage + ((size_t)b * Hq + h) * kHeadDim) + sub) = raw;
         }
-        __syncthreads();  // inputs (and, in the first pass, the weights) are in shared memory
-        int cur = 0;  // which of the two activation buffers holds the input of the next layer
+        if (row < kHmRows) *reinterpret_cast<uint4*>(&sm.x[0][row][sub * 8]) = raw;
+        __syncthreads();
+        // layers: 3 = W0, W1, W2; 2 = W0, W2; 1 = W2
+        float acc[kHmTiles][4], last[1][4];
         if (p.layers >= 2) {
-            hdb_hidden(sm, sm.wt0, sm.bias, cur, tid);
-            cur ^= 1;
+            hm_gemm<1>(acc, sm.x, 0, w0, lane);
+            hm_activate(sm.act[0], acc, b0, warp, lane);
+            __syncthreads();
         }
         if (p.layers == 3) {
-            hdb_hidden(sm, sm.wt1, sm.bias + kHidden, cur, tid);
-            cur ^= 1;
+            hm_gemm<kHmParts>(acc, sm.act[0], 0, w1, lane);
+            hm_activate(sm.act[1], acc, b1, warp, lane);
+            __syncthreads();
         }
-        // ---- last layer: warp = row, lane = output bit
-        float pre = sm.bias[2 * kHidden + lane];
-#pragma unroll 16
-        for (int i = 0; i < kHidden; ++i) pre = fmaf(sm.x[cur][warp][i], sm.wt2[i][lane], pre);
-        // bit i = 1 iff output i > 0 (efficiency/kernels/torchatt.py:35-36: relu(sign(x)))
-        const uint32_t code = __ballot_sync(0xffffffffu, pre > 0.0f);
-        __syncthreads();  // the activation buffers are rewritten by the next pass
-        if (!live) continue;
-        if (p.preact_dbg != nullptr)
-            p.preact_dbg[(((size_t)b * 2 + side) * Hq + h) * kCodeBits + lane] = pre;
-        if (side == 0) {
-            if (lane == 0) p.q_codes[(size_t)b * Hq + h] = code;
-            continue;
+        if (p.layers == 1) hm_gemm<1>(last, sm.x, blk2, w2, lane);
+        else hm_gemm<kHmParts>(last, sm.act[p.layers - 2], blk2, w2, lane);
+        {
+            float(*part)[kCodeBits] = sm.part[warp / 4];
+            const int col = tile2 * 8 + (lane % 4) * 2;
+            *reinterpret_cast<float2*>(&part[lane / 4][col]) = make_float2(last[0][0], last[0][1]);
+            *reinterpret_cast<float2*>(&part[lane / 4 + 8][col]) = make_float2(last[0][2], last[0][3]);
         }
-        if (S < 1 || S > p.max_pages * kPage) {
-            if (lane == 0) report(p.status, HA_ERR_BAD_SEQ_LEN);
-            continue;
+        __syncthreads();
+        // ---- codes: lane = output bit, the warp's two rows; bit i = 1 iff output i > 0 (efficiency/kernels/torchatt.py:35-36:
+        //      relu(sign(x))). Every buffer is written again only behind a barrier that its readers have passed.
+        if (warp >= kHmRows / 2) continue;
+        float pre0 = b2, pre1 = b2;
+#pragma unroll
+        for (int i = 0; i < kSplit; ++i) {
+            pre0 += sm.part[i][2 * warp][lane];
+            pre1 += sm.part[i][2 * warp + 1][lane];
         }
-        if (page < 0 || page >= p.num_pages) {
-            if (lane == 0) report(p.status, HA_ERR_BAD_PAGE);
-            continue;
+        const uint32_t code0 = __ballot_sync(0xffffffffu, pre0 > 0.0f), code1 = __ballot_sync(0xffffffffu, pre1 > 0.0f);
+        const uint32_t code = half == 0 ? code0 : code1;
+        if (p.preact_dbg != nullptr) {
+            const int first = r0 + 2 * warp;
+            if (first < b_end) p.preact_dbg[(((size_t)first * 2 + side) * Hq + h) * kCodeBits + lane] = pre0;
+            if (first + 1 < b_end) p.preact_dbg[(((size_t)(first + 1) * 2 + side) * Hq + h) * kCodeBits + lane] = pre1;
         }
-        const size_t slot = ((size_t)page * p.Hkv + kvh) * kPage + (S - 1) % kPage;
-        if (lane == 0) p.hash_pages[slot * kGroup + g] = code;
-        if (appends) {  // 256 B each
-            uint4* dp = lane < 16 ? reinterpret_cast<uint4*>(p.k_pages + slot * kHeadDim) + lane
-                                  : reinterpret_cast<uint4*>(p.v_pages + slot * kHeadDim) + (lane - 16);
-            *dp = app;
+        if (live && side == 0) {
+            if (sub == 0) p.q_codes[(size_t)b * Hq + h] = code;
+        } else if (live && (S < 1 || S > p.max_pages * kPage)) {
+            if (sub == 0) report(p.status, HA_ERR_BAD_SEQ_LEN);
+        } else if (live && (page < 0 || page >= p.num_pages)) {
+            if (sub == 0) report(p.status, HA_ERR_BAD_PAGE);
+        } else if (live) {
+            const size_t slot = ((size_t)page * p.Hkv + kvh) * kPage + (S - 1) % kPage;
+            if (sub == 0) p.hash_pages[slot * kGroup + g] = code;
+            if (appends) {  // 256 B each
+                *(reinterpret_cast<uint4*>(p.k_pages + slot * kHeadDim) + sub) = raw;
+                *(reinterpret_cast<uint4*>(p.v_pages + slot * kHeadDim) + sub) = v_raw;
+            }
         }
+        __syncwarp();
     }
 }
 

@@ -676,26 +676,13 @@ static int hash_decode_impl(const ha_shape_t* shape, const ha_hash_weights_t* we
     const dim3 grid(shape->num_kv_heads * kGroup, key_side ? 2 : 1,
                     (shape->batch + p.batch_per_cta - 1) / p.batch_per_cta);
     cudaError_t e;
-    if (p.batch_per_cta >= kHdbMinRows) {
-        // several sequences per CTA: evaluate them together from shared-memory weights
-        const bool bf16 = weights->dtype == HA_WEIGHTS_BF16;
-        e = bf16 ? cudaFuncSetAttribute(hash_decode_batched_kernel<__nv_bfloat16>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHdbSmemBytes)
-                 : cudaFuncSetAttribute(hash_decode_batched_kernel<float>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHdbSmemBytes);
-        if (e != cudaSuccess) return HA_ERR_LAUNCH;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(kHashDecodeThreads);
-        cfg.dynamicSmemBytes = kHdbSmemBytes;
-        cfg.stream = static_cast<cudaStream_t>(stream);
-        cudaLaunchAttribute attr1[1];
-        attr1[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr1[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr1;
-        cfg.numAttrs = 1;
-        e = bf16 ? cudaLaunchKernelEx(&cfg, hash_decode_batched_kernel<__nv_bfloat16>, p)
-                 : cudaLaunchKernelEx(&cfg, hash_decode_batched_kernel<float>, p);
+    const bool bf16 = weights->dtype == HA_WEIGHTS_BF16;
+    if (p.batch_per_cta >= (bf16 ? kHmMinRows<__nv_bfloat16> : kHmMinRows<float>)) {
+        // several sequences per CTA: evaluate them together on the tensor cores
+        const cudaStream_t st = static_cast<cudaStream_t>(stream);
+        e = bf16
+                ? launch(hash_decode_batched_kernel<__nv_bfloat16>, grid, dim3(kHmWarps<__nv_bfloat16> * 32), st, 1, p)
+                : launch(hash_decode_batched_kernel<float>, grid, dim3(kHmWarps<float> * 32), st, 1, p);
         return e == cudaSuccess ? HA_OK : HA_ERR_LAUNCH;
     }
     const cudaStream_t st = static_cast<cudaStream_t>(stream);

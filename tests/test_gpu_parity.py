@@ -451,6 +451,36 @@ def test_two_layer_hash_function_in_the_batched_encoder(device):
     run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(8, 1.0 / 8, 8), shuffle_seed=4)
 
 
+@pytest.mark.parametrize("batch,bf16_weights,layers", [(5, True, 3), (9, False, 3), (31, True, 2), (32, False, 3), (33, True, 3),
+                                                       (34, False, 2), (6, True, 1), (35, False, 1)])
+def test_batched_encoder_rows(device, batch, bf16_weights, layers):
+    """The batched encoder at the edges of its tiling: the fewest rows per CTA it is used for (3 with bf16 weights, 5 with
+    fp32 ones), 15 and 16 + 1 (a second pass of one row), a last CTA with fewer rows than the first, every depth of the
+    hash function. Pre-activations, codes and appended rows against the oracle."""
+    Hq, Hkv = 32, 8
+    lens = [1 + (37 * b) % 300 for b in range(batch)]
+    usa = synthetic.make_usa(Hq, 128, 11, bf16_weights, num_layers=layers)
+    inp = synthetic.make_decode_inputs(120 + batch, lens, Hq, Hkv)
+    cache, ctx = build(device, inp.q, inp.k, inp.v, ha.Budget(16, 0.125, 16), usa, prefill_to=[s - 1 for s in lens])
+    cache.seq_lens += 1
+    k_new = torch.stack([k[:, -1] for k in inp.k]).to(device, torch.bfloat16)
+    v_new = torch.stack([v[:, -1] for v in inp.v]).to(device, torch.bfloat16)
+    pre = torch.zeros(batch, 2, Hq, 32, device=device)
+    q_codes = ctx.hash_decode(inp.q.to(device, torch.bfloat16), k_new, v_new, preact_dbg=pre).cpu().to(torch.int64) & ALL_BITS
+    ctx.check_status()
+    worst = 0.0
+    for b in range(batch):
+        q_pre, k_pre = helpers.oracle_preacts(usa, inp.q[b:b + 1], inp.k[b][None, :, -1:, :])
+        assert helpers.codes_match(q_codes[b], orc.pack_codes(q_pre[0]), orc.band_mask(q_pre[0]))
+        assert helpers.codes_match(cache.read_codes(b).cpu()[:, -1], orc.pack_codes(k_pre[0, :, 0]), orc.band_mask(k_pre[0, :, 0]))
+        worst = max(worst, float((pre[b, 0].cpu() - q_pre[0]).abs().max()), float((pre[b, 1].cpu() - k_pre[0, :, 0]).abs().max()))
+        k_back, v_back = cache.read_kv(b)
+        assert torch.equal(k_back.float().cpu(), inp.k[b]) and torch.equal(v_back.float().cpu(), inp.v[b])
+    # half of the exclusion band, as for the other encoder: sums of 128 products of order one in fp32 are off by less than
+    # 128 * 2^-24 = 7.6e-6 even if every rounding goes one way
+    assert worst < 5e-6, f"pre-activation error {worst} would eat into the 1e-5 exclusion band"
+
+
 def test_ragged_batch_shuffled_pages(device):
     Hq, Hkv, lens = 8, 2, [1, 2, 31, 255, 256, 257, 1500, 4097]
     usa = synthetic.make_usa(Hq, 128, 2, True)
