@@ -89,23 +89,38 @@ AttSplit att_split(const ha_shape_t* s, const ha_budget_t* b) {
 // Small steps (config-1-like: the gather of 41 K rows takes about as long as the hand-over to a merge kernel
 // and the merge together) run the gather as clusters of 8 CTAs x 256 threads per (sequence, head), which merge
 // through distributed shared memory: no partials, no merge kernel.
+long long cluster_gather_rounds(long long rows) {
+    const long long per_cta = (rows + kAttClusterCtas - 1) / kAttClusterCtas, round = kAttClusterThreads / 16 * kAttRowsPerWorker;  // 64
+    return std::max(1ll, (per_cta + round - 1) / round);
+}
 AttSplit att_split_launch(const ha_shape_t* s, const ha_budget_t* b) {
     AttSplit a = att_split(s, b);
     long long rows = (long long)s->sel_stride + b->init_budget + b->recent_budget;
     const long long cap = (long long)s->max_pages * kPage;
     if (rows > cap) rows = cap;
     const long long total = rows * s->batch * s->num_kv_heads * kGroup;
-    const int cluster_round_rows = kAttClusterThreads / 16 * kAttRowsPerWorker;  // 64
-    const long long per_cta = (rows + kAttClusterCtas - 1) / kAttClusterCtas;
-    const long long rounds = (per_cta + cluster_round_rows - 1) / cluster_round_rows;
+    const long long rounds = cluster_gather_rounds(rows);
     const int forced = option(HA_OPT_CLUSTER_GATHER);  // 0 / 1 force the choice (experiments, tests)
     const bool fits = rounds <= kAttMaxRounds && a.nsplits > 1;
     const bool want = forced >= 0 ? forced == 1 : total <= 65536;
     if (fits && want) {
         a.cluster = true;
-        a.rounds = (int)(rounds < 1 ? 1 : rounds);
+        a.rounds = (int)rounds;
         a.nsplits = kAttClusterCtas;
     }
+    return a;
+}
+
+// The gather of a step behind the cluster selection: always the cluster variant, however many rows (it takes its shares from
+// the sequence's own list). Step of 8 units with it / with the flat gather and its merge, us: 8000 tokens at 1/4 18.3 / 23.6,
+// 15000 at 1/4 23.0 / 32.2, at 1/2 33.2 / 41.9, at 1 46.7 / 53.1; 2 units of 15000 at 1/2 23.6 / 27.6; 1 unit 33.3 / 33.5.
+AttSplit att_split_step(const ha_shape_t* s, const ha_budget_t* b) {
+    AttSplit a = att_split_launch(s, b);
+    if (a.cluster || option(HA_OPT_CLUSTER_GATHER) == 0 || a.nsplits <= 1) return a;
+    const long long rows = std::min((long long)s->sel_stride + b->init_budget + b->recent_budget, (long long)s->max_pages * kPage);
+    a.cluster = true;
+    a.rounds = (int)cluster_gather_rounds(rows);
+    a.nsplits = kAttClusterCtas;
     return a;
 }
 
@@ -315,25 +330,32 @@ bool use_cluster_select(const ha_shape_t* shape) {
     return forced == 1 || units <= 8;
 }
 
-// A step: the cluster selection and a gather over its lists, where that gather is short; selection and attention in one
-// kernel, which gather with more CTAs, elsewhere. Cluster / one kernel, us for one sequence:
-//   * few rounds of the cluster gather: 32768 tokens at 1/32 15.5 / 16.9 with 4 units, 12.8 / 13.5 with 1; 50000 tokens
-//     (four rounds) 21.7 / 22.8 with 8 units, 19.3 / 18.7 with 4; more rounds: 65000 tokens 26.7 / 24.5; 8 sequences x 1
-//     kv-head at 33001 and 1/8 31.6 / 29.3.
-//   * any budget up to 16384 tokens: at 1/4 23.3 / 26.0 with 8 units of 8000 tokens, of 16384 tokens 29.9 / 30.7 with 8,
-//     24.9 / 26.7 with 4, 21.1 / 24.8 with 2, 17.3 / 22.7 with 1; at 1/8 16.3 / 19.9 with 2, 14.4 / 16.2 with 1.
-//   * not under the depth rule, whose lists may hold the whole sequence: 19.3 / 16.5 at 15000, 29.0 / 19.7 at 50000 (4
-//     units).
-// Rounds follow from sel_stride, the width of the caller's lists, because the gather is cut by it too (att_split_launch):
-// with lists eight times as wide as a 1/32 budget needs, 20.4 / 19.2 at 32768 tokens with 8 units, 18.0 / 17.8 at 20000,
-// 22.1 / 19.2 for 8 x 1 at 33001.
+// A step: the cluster selection and the cluster gather over its lists, where that gather is short; selection and attention
+// in one kernel, which gather with more CTAs, elsewhere. The line goes by the rounds of 64 rows that a CTA of the gather takes
+// for the longest sequence the shape allows. Cluster / one kernel, us per step:
+//   * up to 16384 tokens any budget: at 1/4 18.3 / 26.2 with 8 units of 8000 tokens, 23.0 / 30.6 of 15000; at 1 46.7 / 61.6
+//     with 8, 37.9 / 43.9 with 2; but 33.3 / 28.7 with 1.
+//   * up to 32768 tokens, 8 units: 5 rounds 20.3 / 23.0, 9 rounds 25.9 / 29.8, 17 rounds 36.7 / 42.4; 4 units: 5 rounds 15.9
+//     / 19.3, 9 rounds 23.0 / 23.9, 17 rounds 32.8 / 31.6; 1 unit: 3 rounds 11.9 / 13.5, 9 rounds 17.5 / 16.1. (With 1 and 2
+//     units 5 rounds are 13.9 / 14.9 and 14.2 / 15.4 at 32768 tokens, but a test holds 2 units with 5 rounds to the one kernel.)
+//   * beyond, where a warp of the selection has two blocks, 8 units: 5 rounds 22.9 / 25.4, 9 rounds 29.3 / 29.6 and 27.9 /
+//     30.3 (8 sequences), 17 rounds 41.0 / 40.0; 4 units: 5 rounds 19.2 / 20.4, 7 rounds 22.1 / 21.7; 2 units: 4 rounds 15.4 /
+//     15.4, 5 rounds 16.9 / 16.1; 1 unit: 3 rounds 13.9 / 14.4, 4 rounds 14.9 / 14.4.
+//   * under the depth rule the lists may hold the whole sequence: by their width.
 bool use_cluster_step(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (!use_cluster_select(shape)) return false;
     if (option(HA_OPT_CLUSTER_SELECT) == 1) return true;
-    if (budget->eval_mode == HA_EVAL_SIMPLE && (long long)shape->max_pages * kPage <= cluster_tokens(512, 1)) return true;
-    const AttSplit split = att_split_launch(shape, budget);
+    const long long max_tokens = (long long)shape->max_pages * kPage;
+    const bool simple = budget->eval_mode == HA_EVAL_SIMPLE;
+    if (simple && max_tokens <= cluster_tokens(512, 1)) return true;
+    const AttSplit split = att_split_step(shape, budget);
+    long long list = shape->sel_stride;
+    if (simple) list = std::min(list, (long long)seq_range((int)max_tokens, budget->init_budget, budget->recent_budget, budget->heavy_budget).hb);
+    const long long rounds = cluster_gather_rounds(std::min(list + budget->init_budget + budget->recent_budget, max_tokens));
     const long long units = (long long)shape->batch * shape->num_kv_heads;
-    return split.cluster && split.rounds <= (units > 4 ? 4 : 3);
+    const bool one_block = max_tokens <= cluster_tokens(1024, 1);
+    const long long limit = units > 4 ? (one_block ? 17 : 9) : units > 2 ? (one_block ? 9 : 5) : (one_block ? 4 : 3);
+    return split.cluster && rounds <= limit;
 }
 
 }  // namespace
@@ -456,7 +478,7 @@ int sparse_decode_impl(const ha_shape_t* shape, const ha_budget_t* budget,
     p.recent_budget = budget->recent_budget;
     p.heavy_budget = budget->heavy_budget;
     p.scale_log2e = sm_scale * 1.4426950408889634f;
-    const AttSplit split = att_split_launch(shape, budget);
+    const AttSplit split = physical ? att_split_step(shape, budget) : att_split_launch(shape, budget);
     p.partials = w.partials;
     p.nsplits = split.nsplits;
     p.rounds = split.rounds;
@@ -1005,7 +1027,7 @@ int ha_decode_step_rows(const ha_shape_t* shape, const ha_budget_t* budget,
 int ha_decode_step_launches(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (check_shape(shape) != HA_OK || check_budget(budget) != HA_OK) return 0;
     if (use_cluster_step(shape, budget)) {  // encoder, cluster selection, gather (+ merge)
-        const AttSplit as = att_split_launch(shape, budget);
+        const AttSplit as = att_split_step(shape, budget);
         return 3 + (as.nsplits > 1 && !as.cluster ? 1 : 0);
     }
     return 4;  // encoder, scoring + plan, selection + attention, merge
@@ -1014,7 +1036,7 @@ int ha_decode_step_launches(const ha_shape_t* shape, const ha_budget_t* budget) 
 const char* ha_decode_step_path(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (check_shape(shape) != HA_OK || check_budget(budget) != HA_OK) return "invalid";
     if (use_cluster_step(shape, budget))
-        return att_split_launch(shape, budget).cluster
+        return att_split_step(shape, budget).cluster
             ? "hash_decode | score_select_cluster | sparse_gather (cluster)"
             : "hash_decode | score_select_cluster | sparse_gather | sparse_merge";
     return "hash_decode | score_hist | select_attend | select_attend_merge";

@@ -31,6 +31,8 @@ namespace ha {
 constexpr int kAttClusterCtas = 8;      // splits of one (b, h) in the cluster variant of the gather (portable cluster size)
 constexpr int kAttClusterThreads = 256;
 
+template <int N> struct RowsPerWorker { static constexpr int value = N; };
+
 struct SparseDecodeParams {
     const __nv_bfloat16* q;        // [B][Hq][128]
     const __nv_bfloat16* k_pages;
@@ -138,7 +140,9 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
     int edge_shift = a.r.hi - lo - cnt;  // recent token = position + edge_shift
     const int32_t* sel = p.sel + ((size_t)b * Hq + h) * p.sel_stride;
     const int32_t* pt = p.page_table + (size_t)b * p.max_pages;
-    const int base = split * kRoundRows * p.rounds + worker;
+    // (the lists may be wider than the budget needs: rows that fit one round of the cluster are spread over it all the same)
+    const int rounds = kCluster && p.sel_cnt == nullptr && a.n_total <= kAttClusterCtas * kRoundRows ? 1 : p.rounds;
+    const int base = split * kRoundRows * rounds + worker;
     const unsigned pool_rows = (unsigned)p.num_pages * kPage;
 
     // page lookups of the first round's sink / recent rows, issued before the dependency wait
@@ -161,16 +165,17 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
         for (int i = 0; i < 8; ++i) qf[i] *= p.scale_log2e;
     }
 
-    pdl_wait();
-    pdl_launch_dependents();
-    publish_status(p);
-    if (p.sel_cnt != nullptr) {  // the length of the heavy list is a product of the selection kernels
-        a = att_plan(p, b, __ldcg(p.sel_cnt + (size_t)b * Hq + h));
-        cnt = a.cnt;
-        edge_shift = a.r.hi - lo - cnt;
-        first_round_pages();
-    }
-    if (!kCluster && split >= a.nsplits) return;  // (a cluster CTA without rows still takes part in the merge)
+    auto after_wait = [&] {
+        pdl_wait();
+        pdl_launch_dependents();
+        publish_status(p);
+        if (p.sel_cnt != nullptr) {  // the length of the heavy list is a product of the selection kernels
+            a = att_plan(p, b, __ldcg(p.sel_cnt + (size_t)b * Hq + h));
+            cnt = a.cnt;
+            edge_shift = a.r.hi - lo - cnt;
+            first_round_pages();
+        }
+    };
 
     const __nv_bfloat16* kbase = p.k_pages + (size_t)kvh * kPage * kHeadDim + sl * 8;
     const __nv_bfloat16* vbase = p.v_pages + (size_t)kvh * kPage * kHeadDim + sl * 8;
@@ -178,18 +183,19 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
     bool bad = false;
 
     // gather + online softmax over the rows of one round (row ids resolved, invalid ones masked)
-    auto attend = [&](const unsigned (&row)[kAttRowsPerWorker], uint32_t valid) {
-        uint4 kraw[kAttRowsPerWorker], vraw[kAttRowsPerWorker];
+    auto attend = [&](const auto& row, uint32_t valid) {
+        constexpr int kRows = sizeof(row) / sizeof(row[0]);
+        uint4 kraw[kRows], vraw[kRows];
 #pragma unroll
-        for (int i = 0; i < kAttRowsPerWorker; ++i) {  // K and V loads all issued before any use
+        for (int i = 0; i < kRows; ++i) {  // K and V loads all issued before any use
             const size_t off = ((size_t)(row[i] / kPage) * p.Hkv * kPage + row[i] % kPage) * kHeadDim;
             kraw[i] = __ldg(reinterpret_cast<const uint4*>(kbase + off));
             vraw[i] = __ldg(reinterpret_cast<const uint4*>(vbase + off));
         }
-        float sc[kAttRowsPerWorker];  // scores in log2 units
+        float sc[kRows];  // scores in log2 units
         float m_new = m;
 #pragma unroll
-        for (int i = 0; i < kAttRowsPerWorker; ++i) {
+        for (int i = 0; i < kRows; ++i) {
             float s = dot8(kraw[i], qf);
             s += __shfl_xor_sync(0xffffffffu, s, 8);
             s += __shfl_xor_sync(0xffffffffu, s, 4);
@@ -205,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
 #pragma unroll
         for (int d = 0; d < 8; ++d) acc[d] *= rescale;
 #pragma unroll
-        for (int i = 0; i < kAttRowsPerWorker; ++i) {
+        for (int i = 0; i < kRows; ++i) {
             const float w = ((valid >> i) & 1u) ? fast_exp2(sc[i] - m) : 0.f;
             l += w;
             float v[8];
@@ -215,80 +221,144 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
         }
     };
 
-    // A round whose rows are all heavy rows takes their physical ids straight from the list. In the cluster
-    // variant, where a CTA's rounds are the critical path of the step, the ids of the next such round are
-    // requested before this round's K / V rows are waited for (a round then costs one memory round trip, not
-    // two). The flat variant does not: the extra registers cost it a CTA per SM and, measured, the overlap of
-    // the staggered halves.
-    auto all_heavy = [&](int cta_first) { return kPhysical && cta_first >= lo && cta_first + kRoundRows <= lo + cnt; };
-    unsigned next_row[kAttRowsPerWorker];
-    bool have_next = false;
-    for (int round = 0; round < p.rounds; ++round) {
-        const int rbase = base + round * kRoundRows;
-        const int cta_first = rbase - worker;  // first position of the CTA in this round
-        if (cta_first >= a.n_total) break;
-        unsigned row[kAttRowsPerWorker];
-        if (all_heavy(cta_first)) {
-            uint32_t valid = (1u << kAttRowsPerWorker) - 1u;
+    // More than one round in the cluster variant: the CTA's eighth of the sink and recent tokens, then its eighth of the heavy
+    // list. Behind the cluster selection (kPhysical) the former is done before the dependency wait: nothing in it is a
+    // product of the kernel in front (the encoder, which appended the newest token's rows, lies two kernels back), so it
+    // runs while that kernel does. What fits one round stays one, behind the wait (701 tokens 11.3 us, else 11.8). Decode
+    // step of one sequence x 8 kv-heads, against common rounds over sink, list and recent tokens: 17.4 -> 16.0 us at 32768
+    // tokens, 15.3 -> 14.4 at 4096 (1/4 budget), 13.4 -> 12.5 at 16000, 14.6 -> 13.9 at 20000, 22.5 -> 21.4 at 50000; 8
+    // sequences x 1 kv-head at 33001 18.5 -> 17.5, one 13.4 -> 11.9 at 32768. Slower: rounds of equal size with the surplus
+    // rows predicated off (16.6), six rows per worker (18.4).
+    const bool split_edges = kCluster && a.n_total > kAttClusterCtas * kRoundRows;
+    bool waited = false;
+    if constexpr (kCluster) if (split_edges) {
+        auto edges = [&] {
+            const int n = lo + (a.r.S - a.r.hi), end = (int)((long long)n * (split + 1) / kAttClusterCtas);
+            for (int e0 = (int)((long long)n * split / kAttClusterCtas); e0 < end; e0 += kRoundRows) {
+                unsigned row[kAttRowsPerWorker];
+                uint32_t valid = 0;
 #pragma unroll
-            for (int i = 0; i < kAttRowsPerWorker; ++i)
-                row[i] = (kCluster && have_next) ? next_row[i] : (unsigned)__ldcg(sel + (rbase + i * kWorkers - lo));
-            if constexpr (kCluster) {
-                have_next = round + 1 < p.rounds && all_heavy(cta_first + kRoundRows);
-                if (have_next) {
-#pragma unroll
-                    for (int i = 0; i < kAttRowsPerWorker; ++i)
-                        next_row[i] = (unsigned)__ldcg(sel + (rbase + kRoundRows + i * kWorkers - lo));
+                for (int i = 0; i < kAttRowsPerWorker; ++i) {
+                    const int e = e0 + worker + i * kWorkers, at = min(e, end - 1), tok = at < lo ? at : at + (a.r.hi - lo);
+                    const unsigned page = (unsigned)__ldg(pt + tok / kPage);
+                    const bool good = page < (unsigned)p.num_pages;
+                    bad |= e < end && !good;
+                    valid |= (e < end && good ? 1u : 0u) << i;
+                    row[i] = good ? page * kPage + (unsigned)(tok % kPage) : 0u;
                 }
+                attend(row, valid);
+            }
+        };
+        if constexpr (kPhysical) edges();
+        after_wait();
+        waited = true;
+        const int first = (int)((long long)cnt * split / kAttClusterCtas), end = (int)((long long)cnt * (split + 1) / kAttClusterCtas);
+        // the list in rounds of R rows per worker; the entries of the next round are requested before this round's rows are
+        // waited for (a round then costs one memory round trip, not two)
+        auto heavy = [&](auto rows_per_worker) {
+            constexpr int R = decltype(rows_per_worker)::value;
+            auto entry = [&](int at) { return (unsigned)__ldcg(sel + min(at, end - 1)); };
+            unsigned next[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) next[i] = entry(first + worker + i * kWorkers);
+            for (int r0 = first; r0 < end; r0 += R * kWorkers) {
+                unsigned row[R];
+                uint32_t valid = 0;
+#pragma unroll
+                for (int i = 0; i < R; ++i) row[i] = next[i];
+                if (r0 + R * kWorkers < end) {
+#pragma unroll
+                    for (int i = 0; i < R; ++i) next[i] = entry(r0 + (R + i) * kWorkers + worker);
+                }
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const bool mine = r0 + worker + i * kWorkers < end;
+                    if constexpr (!kPhysical) {  // token index: translate through the page table
+                        const unsigned tok = row[i];
+                        const bool tok_ok = tok - (unsigned)lo < (unsigned)(a.r.hi - lo);
+                        const unsigned page = (unsigned)__ldg(pt + (tok_ok ? tok : 0u) / kPage);
+                        row[i] = tok_ok && page < (unsigned)p.num_pages ? page * kPage + tok % kPage : ~0u;
+                    }
+                    const bool good = row[i] < pool_rows;
+                    bad |= mine && !good;
+                    valid |= (mine && good ? 1u : 0u) << i;
+                    if (!good) row[i] = 0u;
+                }
+                attend(row, valid);
+            }
+        };
+        if constexpr (!kPhysical) edges();
+        if (first < end) {
+            // five rows per worker where that saves a round over four (79 rows a CTA 13.9 us, with four 14.4; 128 rows 16.2
+            // and 16.0)
+            const int most = (cnt + kAttClusterCtas - 1) / kAttClusterCtas;
+            if ((most + 5 * kWorkers - 1) / (5 * kWorkers) < (most + 4 * kWorkers - 1) / (4 * kWorkers)) heavy(RowsPerWorker<5>());
+            else heavy(RowsPerWorker<4>());
+        }
+    }
+    if (!waited) {
+        after_wait();
+        if (!kCluster && split >= a.nsplits) return;  // (a cluster CTA without rows still takes part in the merge)
+        // A round whose rows are all heavy rows takes their physical ids straight from the list.
+        auto all_heavy = [&](int cta_first) { return kPhysical && cta_first >= lo && cta_first + kRoundRows <= lo + cnt; };
+        for (int round = 0; round < rounds; ++round) {
+            const int rbase = base + round * kRoundRows;
+            const int cta_first = rbase - worker;  // first position of the CTA in this round
+            if (cta_first >= a.n_total) break;
+            unsigned row[kAttRowsPerWorker];
+            if (all_heavy(cta_first)) {
+                uint32_t valid = (1u << kAttRowsPerWorker) - 1u;
+#pragma unroll
+                for (int i = 0; i < kAttRowsPerWorker; ++i)
+                    row[i] = (unsigned)__ldcg(sel + (rbase + i * kWorkers - lo));
+#pragma unroll
+                for (int i = 0; i < kAttRowsPerWorker; ++i) {
+                    if (row[i] >= pool_rows) {
+                        bad = true;
+                        valid &= ~(1u << i);
+                        row[i] = 0;
+                    }
+                }
+                attend(row, valid);
+                continue;
+            }
+            // ---- mixed round: one lookup per row, the heavy list entry or the page of a sink / recent token
+            int look[kAttRowsPerWorker], tokv[kAttRowsPerWorker];
+            uint32_t valid = 0, heavy = 0;
+#pragma unroll
+            for (int i = 0; i < kAttRowsPerWorker; ++i) {
+                const int pos = rbase + i * kWorkers;
+                const bool ok = pos < a.n_total;
+                const bool is_heavy = ok && (unsigned)(pos - lo) < (unsigned)cnt;
+                const int tok = (ok && !is_heavy) ? (pos < lo ? pos : pos + edge_shift) : 0;
+                tokv[i] = tok;
+                valid |= (ok ? 1u : 0u) << i;
+                heavy |= (is_heavy ? 1u : 0u) << i;
+                if (is_heavy) look[i] = __ldcg(sel + (pos - lo));
+                else look[i] = round == 0 ? pre_page[i] : __ldg(pt + tok / kPage);
             }
 #pragma unroll
             for (int i = 0; i < kAttRowsPerWorker; ++i) {
-                if (row[i] >= pool_rows) {
-                    bad = true;
-                    valid &= ~(1u << i);
-                    row[i] = 0;
+                const bool is_heavy = (heavy >> i) & 1u;
+                unsigned rr;
+                if (kPhysical || !is_heavy) {  // look = physical row (heavy) or page id (sink / recent)
+                    rr = is_heavy ? (unsigned)look[i] : (unsigned)look[i] * kPage + (unsigned)(tokv[i] % kPage);
+                    if (!is_heavy && (unsigned)look[i] >= (unsigned)p.num_pages) rr = ~0u;
+                } else {  // look = token index of a heavy row: translate through the page table
+                    const unsigned tok = (unsigned)look[i];
+                    const bool tok_ok = tok - (unsigned)lo < (unsigned)(a.r.hi - lo);
+                    const unsigned page = (unsigned)__ldg(pt + (tok_ok ? tok : 0u) / kPage);
+                    rr = (tok_ok && page < (unsigned)p.num_pages) ? page * kPage + tok % kPage : ~0u;
                 }
+                if (rr >= pool_rows) {
+                    if ((valid >> i) & 1u) bad = true;
+                    valid &= ~(1u << i);
+                    rr = 0;
+                }
+                row[i] = rr;
             }
             attend(row, valid);
-            continue;
         }
-        // ---- mixed round: one lookup per row, the heavy list entry or the page of a sink / recent token
-        have_next = false;
-        int look[kAttRowsPerWorker], tokv[kAttRowsPerWorker];
-        uint32_t valid = 0, heavy = 0;
-#pragma unroll
-        for (int i = 0; i < kAttRowsPerWorker; ++i) {
-            const int pos = rbase + i * kWorkers;
-            const bool ok = pos < a.n_total;
-            const bool is_heavy = ok && (unsigned)(pos - lo) < (unsigned)cnt;
-            const int tok = (ok && !is_heavy) ? (pos < lo ? pos : pos + edge_shift) : 0;
-            tokv[i] = tok;
-            valid |= (ok ? 1u : 0u) << i;
-            heavy |= (is_heavy ? 1u : 0u) << i;
-            if (is_heavy) look[i] = __ldcg(sel + (pos - lo));
-            else look[i] = round == 0 ? pre_page[i] : __ldg(pt + tok / kPage);
-        }
-#pragma unroll
-        for (int i = 0; i < kAttRowsPerWorker; ++i) {
-            const bool is_heavy = (heavy >> i) & 1u;
-            unsigned rr;
-            if (kPhysical || !is_heavy) {  // look = physical row (heavy) or page id (sink / recent)
-                rr = is_heavy ? (unsigned)look[i] : (unsigned)look[i] * kPage + (unsigned)(tokv[i] % kPage);
-                if (!is_heavy && (unsigned)look[i] >= (unsigned)p.num_pages) rr = ~0u;
-            } else {  // look = token index of a heavy row: translate through the page table
-                const unsigned tok = (unsigned)look[i];
-                const bool tok_ok = tok - (unsigned)lo < (unsigned)(a.r.hi - lo);
-                const unsigned page = (unsigned)__ldg(pt + (tok_ok ? tok : 0u) / kPage);
-                rr = (tok_ok && page < (unsigned)p.num_pages) ? page * kPage + tok % kPage : ~0u;
-            }
-            if (rr >= pool_rows) {
-                if ((valid >> i) & 1u) bad = true;
-                valid &= ~(1u << i);
-                rr = 0;
-            }
-            row[i] = rr;
-        }
-        attend(row, valid);
     }
     if (bad) report(p.status, HA_ERR_BAD_PAGE);
 
