@@ -341,7 +341,10 @@ bool use_cluster_select(const ha_shape_t* shape) {
 //   * beyond, where a warp of the selection has two blocks, 8 units: 5 rounds 22.9 / 25.4, 9 rounds 29.3 / 29.6 and 27.9 /
 //     30.3 (8 sequences), 17 rounds 41.0 / 40.0; 4 units: 5 rounds 19.2 / 20.4, 7 rounds 22.1 / 21.7; 2 units: 4 rounds 15.4 /
 //     15.4, 5 rounds 16.9 / 16.1; 1 unit: 3 rounds 13.9 / 14.4, 4 rounds 14.9 / 14.4.
-//   * under the depth rule the lists may hold the whole sequence: by their width.
+//   * under the depth rule the lists may hold the whole sequence: by their width. One sequence at a 1/32 budget: 4096 tokens
+//     12.8 / 14.4 with 8 units, 11.8 / 13.9 with 4; 8192 tokens 13.3 / 14.9 with 8 (at 1/4 19.2 / 27.0). Beyond the limits the
+//     lists decide, which the shape does not know: 30000 tokens 19.2 / 20.7 with 8 units, 15.7 / 17.0 with 4, but 26.8 / 23.7
+//     with 4 at 1/8; 50000 tokens 25.3 / 25.3 and 40.9 / 33.9 with 8.
 bool use_cluster_step(const ha_shape_t* shape, const ha_budget_t* budget) {
     if (!use_cluster_select(shape)) return false;
     if (option(HA_OPT_CLUSTER_SELECT) == 1) return true;

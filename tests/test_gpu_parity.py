@@ -359,6 +359,56 @@ def test_depth_rule_on_the_scoring_plus_fused_selection_path(device, depth):
     assert torch.equal(out0, out1) and torch.equal(ctx0.sel_cnt, ctx1.sel_cnt)
 
 
+@pytest.mark.parametrize("lens,hkv,init", [([4096], 8, 128), ([8192], 8, 128), ([2100, 8000], 4, 128), ([2200, 300], 4, 64),
+                                           ([4500], 3, 128)])
+def test_depth_rule_through_the_cluster_gather(device, lens, hkv, init):
+    """Steps of up to 8 units under the depth rule, by the library's own choice: budgets that predict one round of the cluster
+    (512 rows) or exactly that with ties beyond it, longer lists, and sequences on both sides of 512 rows."""
+    usa = synthetic.make_usa(4 * hkv, 128, 3, True)
+    inp = synthetic.make_decode_inputs(130 + hkv, lens, 4 * hkv, hkv)
+    _, _, ctx, _ = run_step_and_check(device, usa, inp.q, inp.k, inp.v, ha.Budget(init, 1.0 / 32, 128, "depth", 6), shuffle_seed=9)
+    assert "score_select_cluster" in ctx.step_path()
+
+
+def test_depth_rule_step_is_not_slower_than_the_path_it_was_preferred_to(device, lib_option):
+    """8192 tokens x 8 kv-heads: the rows of a list much wider than what it holds are spread over the whole cluster. Cut by
+    the lists' width, where CTA 0 had nearly all of them, the step took 1.66 times as long as with selection and attention in
+    one kernel; spread, 0.89 times."""
+    cache = ha.PagedHashKVCache(1, 8, 8192, device, shuffle_seed=3)
+    synthetic.fill_cache_on_device(cache, [8192], seed=3)
+    ctx = ha.SparseDecodeContext(cache, ha.Budget(128, 1.0 / 32, 128, "depth", 6), synthetic.make_usa(32, 128, 3, True).packed(device))
+    ctx.hash_prefill()
+    q = torch.randn(1, 32, 128, device=device).bfloat16()
+    k, v = torch.randn(2, 1, 8, 128, device=device).bfloat16()
+    out = torch.empty_like(q)
+
+    def step_us():
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+            for _ in range(20):
+                ctx.decode_step(q, k, v, out=out)
+        times = []
+        for _ in range(20):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end) * 50.0)
+        return min(times[5:])
+
+    ctx.decode_step(q, k, v, out=out)  # (whatever the library sets up at first use)
+    torch.cuda.synchronize()
+    assert "cluster" in ctx.step_path()
+    own = step_us()
+    lib_option("cluster_select", 0)
+    ctx.decode_step(q, k, v, out=out)
+    torch.cuda.synchronize()
+    other = step_us()
+    ctx.check_status()
+    assert own < 1.2 * other, (own, other)
+
+
 @pytest.mark.parametrize("cluster_select", [-1, 0])
 @pytest.mark.parametrize("name", ["q5", "q16_page", "q3_short", "q4_depth"])
 def test_multi_token_decode_rows_against_reference_output(device, lib_option, name, cluster_select, record_property):
