@@ -872,6 +872,34 @@ def test_host_buffer_entry_point_equals_device_entry_point(device):
     assert torch.equal(out_dev, out_paged)  # pageable buffers: staged through device copies
 
 
+@pytest.mark.parametrize("batch,bf16_weights", [(5, True), (16, True), (33, True), (9, False)])
+def test_host_buffers_of_a_batch_that_takes_the_batched_encoder(device, batch, bf16_weights):
+    """Page-locked rows read over the bus by the batched encoder (3 rows per CTA with bf16 weights, 5 with fp32 ones, and
+    more than one pass): the same bits as from device memory and through staging copies."""
+    Hq, Hkv = 32, 8
+    lens = [1 + (53 * b) % 200 for b in range(batch)]
+    usa = synthetic.make_usa(Hq, 128, 11, bf16_weights)
+    inp = synthetic.make_decode_inputs(140 + batch, lens, Hq, Hkv)
+    k_new = torch.stack([k[:, -1] for k in inp.k]).to(torch.bfloat16)
+    v_new = torch.stack([v[:, -1] for v in inp.v]).to(torch.bfloat16)
+    results = []
+    for pinned in (None, True, False):
+        cache, ctx = build(device, inp.q, inp.k, inp.v, ha.Budget(16, 0.125, 16), usa, prefill_to=[s - 1 for s in lens])
+        ctx.hash_prefill()
+        cache.seq_lens += 1
+        if pinned is None:
+            out = ctx.decode_step(inp.q.to(device, torch.bfloat16), k_new.to(device), v_new.to(device)).cpu()
+        else:
+            buf = ha.HostStepBuffers(ctx, pinned=pinned)
+            buf.q_host.copy_(inp.q.to(torch.bfloat16)); buf.k_host.copy_(k_new); buf.v_host.copy_(v_new)
+            out = ha.decode_step_host(ctx, buf).clone()
+        ctx.check_status()
+        results.append((out, ctx.q_codes.cpu(), cache.hash_pages.cpu(), cache.k_pages.cpu(), cache.v_pages.cpu()))
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
+
+
 def test_host_buffer_step_replayed_as_a_graph(device):
     """decode_step_host(use_graph=True): the recorded call reads the host buffers and the sequence
     lengths at replay time, so consecutive tokens with new inputs come out as from eager calls."""
