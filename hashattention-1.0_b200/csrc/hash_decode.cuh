@@ -593,6 +593,14 @@ __device__ __forceinline__ void hm_activate(__nv_bfloat16 (*dst)[kHmRows][kHmPit
     }
 }
 
+// Eight elements of an input row. Rows handed over for their codes alone may lie on 8-byte boundaries (the branch goes the
+// same way in every thread); where K and V are appended, or attention follows, all tensors lie on 16-byte ones.
+__device__ __forceinline__ uint4 hm_load16(const __nv_bfloat16* p) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return *reinterpret_cast<const uint4*>(p);
+    const uint2 lo = *reinterpret_cast<const uint2*>(p), hi = *reinterpret_cast<const uint2*>(p + 4);
+    return make_uint4(lo.x, lo.y, hi.x, hi.y);
+}
+
 template <typename WT>
 __global__ void __launch_bounds__(kHmWarps<WT> * 32, 1) hash_decode_batched_kernel(const HashDecodeParams p) {
     constexpr int kHmTiles = kHidden / (8 * kHmWarps<WT>);  // n-tiles per warp in a hidden layer: 2 or 1
@@ -624,8 +632,9 @@ __global__ void __launch_bounds__(kHmWarps<WT> * 32, 1) hash_decode_batched_kern
             w0[n][k].load(src + k * 32);
             w1[n][k].load(src + kHidden * kHeadDim + k * 32);
         }
-        b0[n] = __ldg(reinterpret_cast<const float2*>(bias + row) + lane % 4);
-        b1[n] = __ldg(reinterpret_cast<const float2*>(bias + kHidden + row) + lane % 4);
+        const float* b = bias + row + (lane % 4) * 2;  // (biases may lie on any word: single loads)
+        b0[n] = make_float2(__ldg(b), __ldg(b + 1));
+        b1[n] = make_float2(__ldg(b + kHidden), __ldg(b + kHidden + 1));
     }
 #pragma unroll
     for (int k = 0; k < kHmBlocks / kSplit; ++k)
@@ -657,7 +666,7 @@ __global__ void __launch_bounds__(kHmWarps<WT> * 32, 1) hash_decode_batched_kern
         uint4 raw = make_uint4(0u, 0u, 0u, 0u), v_raw = raw;
         int S = 1, page = 0;
         if (live) {
-            raw = *(reinterpret_cast<const uint4*>(x_row(b)) + sub);
+            raw = hm_load16(x_row(b) + sub * 8);
             if (appends) v_raw = *(reinterpret_cast<const uint4*>(p.v_new + ((size_t)b * p.Hkv + kvh) * kHeadDim) + sub);
             if (side == 1) {
                 S = p.seq_lens[b];

@@ -531,6 +531,40 @@ def test_batched_encoder_rows(device, batch, bf16_weights, layers):
     assert worst < 5e-6, f"pre-activation error {worst} would eat into the 1e-5 exclusion band"
 
 
+@pytest.mark.parametrize("bf16_weights", [True, False])
+def test_batched_encoder_takes_rows_on_8_byte_and_biases_on_4_byte_boundaries(device, bf16_weights):
+    """Codes alone (no K / V rows are appended) of tensors that start 8 bytes behind a 16-byte boundary, with biases that
+    start 4 bytes behind one: the same codes as from aligned copies."""
+    batch, Hq, Hkv = 60, 32, 8
+    lens = [1 + (29 * b) % 200 for b in range(batch)]
+    usa = synthetic.make_usa(Hq, 128, 11, bf16_weights)
+    inp = synthetic.make_decode_inputs(150, lens, Hq, Hkv)
+
+    def shifted(t, elements):
+        buf = torch.zeros(t.numel() + 16, dtype=t.dtype, device=device)
+        view = buf[elements:elements + t.numel()].view(t.shape)
+        view.copy_(t)
+        assert view.is_contiguous() and view.data_ptr() % 16 == elements * t.element_size()
+        return view
+
+    q = inp.q.to(device, torch.bfloat16)
+    k = torch.stack([k[:, -1] for k in inp.k]).to(device, torch.bfloat16)
+    results = []
+    for shift in (False, True):
+        cache, ctx = build(device, inp.q, inp.k, inp.v, ha.Budget(16, 0.125, 16), usa)
+        if shift:
+            ctx.weights = copy.copy(ctx.weights)
+            ctx.weights.bq, ctx.weights.bk = shifted(ctx.weights.bq, 1), shifted(ctx.weights.bk, 1)
+            ctx.c_weights = ctx.weights.c_struct(None)
+            q, k = shifted(q, 4), shifted(k, 4)
+        codes = [ctx.hash_decode(q).clone()]
+        codes += [ctx.hash_decode(q, k).clone(), cache.hash_pages.clone()]
+        ctx.check_status()
+        results.append(codes)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 def test_ragged_batch_shuffled_pages(device):
     Hq, Hkv, lens = 8, 2, [1, 2, 31, 255, 256, 257, 1500, 4097]
     usa = synthetic.make_usa(Hq, 128, 2, True)
