@@ -467,7 +467,6 @@ constexpr int kHmRows = 16;             // sequences per CTA and pass
 template <typename WT> constexpr int kHmWarps = sizeof(WT) == 4 ? 16 : 8;
 constexpr int kHmBlocks = kHidden / 32;             // blocks of 32 inputs: 4
 constexpr int kHmParts = 3;             // bf16 parts of an activation
-constexpr float kHmLargest = 3.3895313892515355e38f;
 constexpr int kHmPitch = kHidden + 32;  // elements: 16-byte reads of two neighbouring rows hit different banks
 // Sequences per CTA from which the batched kernel is used. One encoder with 8 kv-heads (two CTAs per head and side), this
 // kernel / the one above, us: bf16 weights 4.5 / 3.9 with 2 rows per CTA, 4.5 / 5.4 with 3, 4.4 / 6.2 with 4, 4.4 / 7.7 with
@@ -574,7 +573,8 @@ __device__ __forceinline__ void hm_gemm(float (&acc)[TILES][4], const __nv_bfloa
         for (int i = 0; i < 4; ++i) acc[n][i] += small[0][n][i] + small[1][n][i];
 }
 
-// bias + SiLU of a hidden layer's accumulators -> the next layer's input, in three bf16 parts
+// bias + SiLU of a hidden layer's accumulators -> the next layer's input, in three bf16 parts. (An activation that is not
+// finite has a NaN among its parts, with which every sum of the row becomes one.)
 template <int TILES>
 __device__ __forceinline__ void hm_activate(__nv_bfloat16 (*dst)[kHmRows][kHmPitch], const float (&acc)[TILES][4],
                                             const float2 (&bias)[TILES], int warp, int lane) {
@@ -584,13 +584,41 @@ __device__ __forceinline__ void hm_activate(__nv_bfloat16 (*dst)[kHmRows][kHmPit
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             uint32_t w[3];
-            // (an infinite activation has no parts: it is held at the largest bf16; a NaN stays one)
-            const float y0 = silu(acc[n][2 * half] + bias[n].x), y1 = silu(acc[n][2 * half + 1] + bias[n].y);
-            split3(y0 > kHmLargest ? kHmLargest : y0, y1 > kHmLargest ? kHmLargest : y1, w);
+            split3(silu(acc[n][2 * half] + bias[n].x), silu(acc[n][2 * half + 1] + bias[n].y), w);
 #pragma unroll
             for (int s = 0; s < kHmParts; ++s) *reinterpret_cast<uint32_t*>(&dst[s][lane / 4 + 8 * half][col]) = w[s];
         }
     }
+}
+
+// The hash function of one row by one warp in plain fp32, lane = output bit; `h`: 256 floats of scratch. For the rows that
+// the matrix form cannot take, because a layer overflows, or the row or the weights hold an infinity or a NaN: they end in
+// sums that are not finite (see hm_activate), which is looked for in the last layer alone and costs the others nothing (32
+// sequences 4.25 us, without it 4.24; with a mark per row and hidden layer 4.41).
+template <typename WT>
+__device__ __forceinline__ float hm_plain_row(const __nv_bfloat16* x, float* h, const WT* W, const float* bias, int layers, int lane) {
+    auto row = [&](const float* in, const WT* w, float b) {
+        float s = 0.f;
+#pragma unroll 1
+        for (int i = 0; i < kHidden; ++i) s = fmaf(in[i], (float)w[i], s);
+        return s + b;
+    };
+    float *in = h, *next = h + kHidden;
+#pragma unroll 1
+    for (int i = lane; i < kHidden; i += 32) in[i] = __bfloat162float(x[i]);
+    __syncwarp();
+#pragma unroll 1
+    for (int l = 0; l < layers - 1; ++l) {  // W0, or W0 and W1
+#pragma unroll 1
+        for (int o = lane; o < kHidden; o += 32) next[o] = silu(row(in, W + (l * kHidden + o) * kHidden, __ldg(bias + l * kHidden + o)));
+        __syncwarp();
+        float* t = in;
+        in = next;
+        next = t;
+    }
+    const float pre = row(in, W + (2 * kHidden + lane) * kHidden, __ldg(bias + 2 * kHidden + lane));
+    __syncwarp();
+    return pre;
 }
 
 // Eight elements of an input row. Rows handed over for their codes alone may lie on 8-byte boundaries (the branch goes the
@@ -705,6 +733,13 @@ __global__ void __launch_bounds__(kHmWarps<WT> * 32, 1) hash_decode_batched_kern
         for (int i = 0; i < kSplit; ++i) {
             pre0 += sm.part[i][2 * warp][lane];
             pre1 += sm.part[i][2 * warp + 1][lane];
+        }
+        if (__any_sync(0xffffffffu, !isfinite(pre0) || !isfinite(pre1))) {
+            // (the activations have been read: this warp's share of their place, until it reaches the next pass's barrier)
+            float* scratch = reinterpret_cast<float*>(&sm.act) + warp * 2 * kHidden;
+            static_assert(sizeof(sm.act) >= kHmRows / 2 * 2 * kHidden * sizeof(float), "scratch of the first eight warps");
+            if (__any_sync(0xffffffffu, !isfinite(pre0))) pre0 = hm_plain_row(sm.x[0][2 * warp], scratch, W, bias, p.layers, lane);
+            if (__any_sync(0xffffffffu, !isfinite(pre1))) pre1 = hm_plain_row(sm.x[0][2 * warp + 1], scratch, W, bias, p.layers, lane);
         }
         const uint32_t code0 = __ballot_sync(0xffffffffu, pre0 > 0.0f), code1 = __ballot_sync(0xffffffffu, pre1 > 0.0f);
         const uint32_t code = half == 0 ? code0 : code1;

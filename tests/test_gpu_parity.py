@@ -565,6 +565,64 @@ def test_batched_encoder_takes_rows_on_8_byte_and_biases_on_4_byte_boundaries(de
         assert torch.equal(a, b)
 
 
+def _rows_with_odd_values(batch, gen, large):
+    """Finite rows with, at known places, infinities of both signs, a NaN and (``large``) values next to the largest ones."""
+    x = torch.randn(batch, 128, generator=gen)
+    x[:, 9].clamp_(-0.5, 0.5)  # (times the largest weight: finite, or what it is added to would decide between inf and NaN)
+    inf, big = float("inf"), 3.0e38
+    rows = [([5], [inf]), ([77], [-inf]), ([5, 6], [inf, -inf]), ([40], [float("nan")])]
+    if large:
+        rows += [([1, 2, 3], [big] * 3), ([20, 21], [-big] * 2), (list(range(128)), [big] * 128)]
+    for i, (places, values) in enumerate(rows):
+        x[2 * i + 1, places] = torch.tensor(values)
+    return x
+
+
+@pytest.mark.parametrize("signed", [True, False])
+@pytest.mark.parametrize("bf16_weights,layers", [(True, 3), (False, 3), (True, 2), (False, 2), (True, 1), (False, 1)])
+def test_batched_encoder_on_values_that_are_not_finite(device, bf16_weights, layers, signed):
+    """Rows whose layers overflow or meet an infinity or a NaN give the codes that the encoder of single rows gives them, and
+    the rows beside them stay as they are. Weights of both signs, and all positive (an infinite sum then stays infinite from
+    layer to layer instead of ending as a NaN, and sums overflow in every order of their terms); per head as they are, with
+    few mantissa bits, with infinities among them, with one next to the largest value."""
+    batch, Hq, Hkv = 20, 8, 2
+    usa = synthetic.make_usa(Hq, 128, 11, bf16_weights, num_layers=layers)
+    with torch.no_grad():
+        for side in (usa.learning_to_hash_transformation_q, usa.learning_to_hash_transformation_k):
+            for h, net in enumerate(side):
+                for lin in [m for m in net if hasattr(m, "weight")]:
+                    if not signed:
+                        lin.weight.abs_()
+                    if h % 4 == 1:
+                        lin.weight.copy_((lin.weight * 8).round().clamp(min=1.0 if not signed else -8.0) / 8)
+                    if h % 4 == 2:
+                        lin.weight[3, 17], lin.weight[20, 64] = float("inf"), -float("inf")
+                    if h % 4 == 3 and not bf16_weights:
+                        lin.weight[4, 9] = 3.4e38
+    gen = torch.Generator().manual_seed(7)
+    q = torch.stack([_rows_with_odd_values(batch, gen, not signed) for _ in range(Hq)], dim=1).to(device, torch.bfloat16)
+    k = torch.stack([_rows_with_odd_values(batch, gen, not signed) for _ in range(Hkv)], dim=1).to(device, torch.bfloat16)
+    cache = ha.PagedHashKVCache(batch, Hkv, 300, device, shuffle_seed=3)
+    cache.seq_lens.fill_(1)
+    ctx = ha.SparseDecodeContext(cache, ha.Budget(16, 0.125, 16), usa.packed(device))
+    # one sequence per CTA: the encoder of single rows
+    one = ha.PagedHashKVCache(1, Hkv, 300, device, shuffle_seed=3)
+    one.seq_lens.fill_(1)
+    single = ha.SparseDecodeContext(one, ha.Budget(16, 0.125, 16), usa.packed(device))
+    many = 8  # the batched encoder is used from 3 (5) sequences per CTA on: the rows are repeated
+    big_cache = ha.PagedHashKVCache(batch * many, Hkv, 300, device, shuffle_seed=3)
+    big_cache.seq_lens.fill_(1)
+    big_ctx = ha.SparseDecodeContext(big_cache, ha.Budget(16, 0.125, 16), usa.packed(device))
+    got_q = big_ctx.hash_decode(q.repeat(many, 1, 1), k.repeat(many, 1, 1)).cpu()
+    big_ctx.check_status()
+    for b in range(batch):
+        want_q = single.hash_decode(q[b:b + 1].contiguous(), k[b:b + 1].contiguous()).cpu()[0]
+        want_k = one.read_codes(0).cpu()[:, 0]
+        for copy_of in (b, b + 5 * batch):
+            assert torch.equal(got_q[copy_of], want_q), (b, (got_q[copy_of] ^ want_q).tolist())
+            assert torch.equal(big_cache.read_codes(copy_of).cpu()[:, 0], want_k), b
+
+
 def test_ragged_batch_shuffled_pages(device):
     Hq, Hkv, lens = 8, 2, [1, 2, 31, 255, 256, 257, 1500, 4097]
     usa = synthetic.make_usa(Hq, 128, 2, True)
