@@ -452,12 +452,12 @@ hash_decode_kernel(const HashDecodeParams p) {
 // free, so a lane's share of 32 inputs is 8 consecutive ones: one 16-byte load each of weights and activations feeds two
 // k-steps.
 // Precision: products of two bf16 are exact. An activation is split into three bf16 (24 bits of mantissa), an fp32 weight
-// too, and products below 2^-24 of the largest are left out. The products of the leading parts are summed up by the
-// matrix instruction over 16 inputs only and from there in fp32 additions, so that its truncation stays below theirs.
-// Pre-activations against a 64-bit evaluation, 100 sequences x 32 heads x 2 sides: rms 11e-9 (bf16 weights) and 17e-9
-// (fp32); with fp32 multiply-adds from transposed fp32 weights in shared memory, the form before, 26e-9 and 27e-9.
+// too; of their nine products the three smallest are left out, the larger two of them at most 2^-22 of the whole each (cut
+// off parts lie below 2^-7 and 2^-15 of it). The products of the leading parts are summed up by the matrix instruction over
+// 16 inputs only and from there in fp32 additions, so that its truncation stays below theirs. Errors of the
+// pre-activations against 64 bits, beside those of the encoder above: at hm_min_rows.
 // What bounds it: latencies - weights, rows, three GEMMs with a barrier each - at about a third of the issue slots. Against
-// that form, whose multiply-adds from shared memory took 3/4 of its time: 12 - 32 sequences x 8 kv-heads 10.9 -> 4.6 us, 64
+// the form before, whose fp32 multiply-adds from transposed fp32 weights in shared memory took 3/4 of its time: 12 - 32 sequences x 8 kv-heads 10.9 -> 4.6 us, 64
 // 18.5 -> 8.0, 100 32.5 -> 14.0; fp32 weights 13.4 -> 8.0 (with parts rounded by cvt instead of truncated 9.5), 21.1 ->
 // 13.6 and 36.0 -> 24.2. With 16 warps for bf16 weights 4.65 and 8.5.
 // ------------------------------------------------------------------------------------------
@@ -470,8 +470,11 @@ constexpr int kHmParts = 3;             // bf16 parts of an activation
 constexpr int kHmPitch = kHidden + 32;  // elements: 16-byte reads of two neighbouring rows hit different banks
 // Sequences per CTA from which the batched kernel is used. One encoder with 8 kv-heads (two CTAs per head and side), this
 // kernel / the one above, us: bf16 weights 4.5 / 3.9 with 2 rows per CTA, 4.5 / 5.4 with 3, 4.4 / 6.2 with 4, 4.4 / 7.7 with
-// 5; fp32 weights 8.0 / 7.1 with 4, 8.0 / 8.7 with 5.
-template <typename WT> constexpr int kHmMinRows = sizeof(WT) == 4 ? 5 : 3;
+// 5; fp32 weights 8.0 / 7.1 with 4, 8.0 / 8.7 with 5. But up to 5 rows, where the kernel above is the alternative, only where
+// the sums are no further from 64 bits than there, rms in units of 1e-9: bf16 weights 7.2 / 7.6 with three layers, 17.5 / 18.8
+// with two, 28.6 / 26.9 with one; fp32 weights 10.8 / 8.6, 24.1 / 23.0, 34.2 / 46.6. (The form before this one had 19.9,
+// 41.9, 39.5 and 20.6, 46.0, 118.)
+inline int hm_min_rows(bool bf16_weights, int layers) { return bf16_weights && layers >= 2 ? 3 : 6; }
 struct HmSmem {
     __align__(16) __nv_bfloat16 x[1][kHmRows][kHmPitch];
     __align__(16) __nv_bfloat16 act[2][kHmParts][kHmRows][kHmPitch];

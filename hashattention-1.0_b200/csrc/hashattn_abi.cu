@@ -702,7 +702,7 @@ static int hash_decode_impl(const ha_shape_t* shape, const ha_hash_weights_t* we
                     (shape->batch + p.batch_per_cta - 1) / p.batch_per_cta);
     cudaError_t e;
     const bool bf16 = weights->dtype == HA_WEIGHTS_BF16;
-    if (p.batch_per_cta >= (bf16 ? kHmMinRows<__nv_bfloat16> : kHmMinRows<float>)) {
+    if (p.batch_per_cta >= hm_min_rows(bf16, p.layers)) {
         // several sequences per CTA: evaluate them together on the tensor cores
         const cudaStream_t st = static_cast<cudaStream_t>(stream);
         e = bf16
