@@ -245,6 +245,105 @@ def test_sparse_attention_matches_reference(device, cases, name):
     assert ok, f"{name}: max_abs={max_abs:.3e} rel_l2={rel:.3e}"
 
 
+def _plain_inputs(seed, lens, hq, hkv):
+    """q, and lists of k / v [Hkv, S, 128], all bf16 values; scores of order 1/4, so that every attended row counts: one row of n
+    too many, too few or exchanged moves a head's output by about 1 / sqrt(n) of its length, 4e-2 at 640 rows."""
+    gen = torch.Generator().manual_seed(seed)
+    q = (0.25 * torch.randn(len(lens), hq, 128, generator=gen)).bfloat16().float()
+    k = [torch.randn(hkv, s, 128, generator=gen).bfloat16().float() for s in lens]
+    v = [torch.randn(hkv, s, 128, generator=gen).bfloat16().float() for s in lens]
+    return q, k, v
+
+
+# what the rounding of the result to bf16 alone can do, 2^-9 of every value, and a little for sums of a few thousand terms
+# in fp32 (2^-24 each)
+GATHER_REL_L2 = 2.0 ** -9 + 1e-4
+
+# list entries per head, sink and recent tokens. Shares of a CTA of the cluster: 1, 64, 65, 79, 80 and 81 list entries; fewer
+# entries than CTAs and none; fewer than eight sink and recent tokens and none; both sides of 512 rows in all
+GATHER_LISTS = [(8, 300, 300), (512, 1, 2), (520, 1, 2), (632, 8, 0), (640, 0, 0), (648, 3, 4), (5, 400, 200), (0, 400, 300),
+                (509, 1, 2), (510, 1, 2), (1100, 64, 64)]
+
+
+@pytest.mark.parametrize("cluster", [1, 0])
+@pytest.mark.parametrize("n,init,recent", GATHER_LISTS)
+def test_gather_over_given_lists(device, lib_option, cluster, n, init, recent):
+    """ha_sparse_decode over lists in any order, cluster form and flat form: a long sequence, one whose candidates end before
+    the budget does, and one that fits one round of the cluster."""
+    lib_option("cluster_gather", cluster)
+    lens = [1500, 900, 400]
+    q, ks, vs = _plain_inputs(31 + n, lens, 8, 2)
+    usa = synthetic.make_usa(8, 128, 0, True)
+    cache, ctx = build(device, q, ks, vs, ha.Budget(init, float(n) if n > 1 else 0.0, recent), usa)
+    gen = torch.Generator().manual_seed(n)
+    sel_idx = torch.zeros_like(ctx.sel_idx, device="cpu")
+    masks = []
+    for b, S in enumerate(lens):
+        lo, hi = min(init, S), max(min(init, S), S - recent)
+        mask = torch.zeros(1, 8, S, dtype=torch.bool)
+        mask[:, :, :lo] = True
+        mask[:, :, hi:] = True
+        for h in range(8):
+            chosen = lo + torch.randperm(hi - lo, generator=gen)[:n]
+            sel_idx[b, h, :len(chosen)] = chosen.to(torch.int32)
+            mask[0, h, chosen] = True
+        masks.append(mask)
+    out = ctx.sparse_decode(q.to(device, torch.bfloat16), sel_idx=sel_idx.to(device)).float().cpu()
+    ctx.check_status()
+    for b in range(len(lens)):
+        ref = orc.masked_attention(q[b:b + 1], ks[b][None], vs[b][None], masks[b])
+        rel = (out[b] - ref[0]).norm(dim=-1) / ref[0].norm(dim=-1)
+        assert float(rel.max()) < GATHER_REL_L2, (b, rel.tolist())
+
+
+@pytest.mark.parametrize("cluster", [1, 0])
+@pytest.mark.parametrize("budget", [64, 900])
+def test_gather_over_given_lists_of_any_length(device, lib_option, cluster, budget):
+    """The same with a length per list (the depth rule), budgets that predict one round and two: none, a few, one round and
+    several, in one call."""
+    lib_option("cluster_gather", cluster)
+    lens, counts = [1500, 1400], [0, 3, 64, 383, 384, 385, 900, 1200]
+    q, ks, vs = _plain_inputs(77, lens, 8, 2)
+    usa = synthetic.make_usa(8, 128, 0, True)
+    cache, ctx = build(device, q, ks, vs, ha.Budget(64, float(budget), 64, "depth", 2), usa)
+    gen = torch.Generator().manual_seed(5)
+    sel_idx, sel_cnt = torch.zeros_like(ctx.sel_idx, device="cpu"), torch.zeros_like(ctx.sel_cnt, device="cpu")
+    masks = []
+    for b, S in enumerate(lens):
+        mask = torch.zeros(1, 8, S, dtype=torch.bool)
+        mask[:, :, :64] = True
+        mask[:, :, S - 64:] = True
+        for h in range(8):
+            chosen = 64 + torch.randperm(S - 128, generator=gen)[:counts[(h + b) % 8]]
+            sel_idx[b, h, :len(chosen)] = chosen.to(torch.int32)
+            sel_cnt[b, h] = len(chosen)
+            mask[0, h, chosen] = True
+        masks.append(mask)
+    out = ctx.sparse_decode(q.to(device, torch.bfloat16), sel_idx=sel_idx.to(device), sel_cnt=sel_cnt.to(device)).float().cpu()
+    ctx.check_status()
+    for b in range(len(lens)):
+        ref = orc.masked_attention(q[b:b + 1], ks[b][None], vs[b][None], masks[b])
+        rel = (out[b] - ref[0]).norm(dim=-1) / ref[0].norm(dim=-1)
+        assert float(rel.max()) < GATHER_REL_L2, (b, rel.tolist())
+
+
+@pytest.mark.parametrize("n,init,recent", [g for g in GATHER_LISTS if g[0] > 1])
+def test_step_through_the_cluster_gather(device, n, init, recent):
+    """The same list lengths through the step, where the gather reads the rows the cluster selection left and attends the sink
+    and recent tokens ahead of it. Sets and outputs against the oracle, the outputs at the bound of the lists' test."""
+    lens = [1500, 900, 400]
+    q, ks, vs = _plain_inputs(31 + n, lens, 8, 2)
+    usa = synthetic.make_usa(8, 128, 3, True)
+    _, out, ctx, cache = run_step_and_check(device, usa, q, ks, vs, ha.Budget(init, float(n), recent))
+    assert ctx.step_path().endswith("sparse_gather (cluster)")
+    q_codes = ctx.q_codes.cpu().to(torch.int64) & ALL_BITS
+    for b, S in enumerate(lens):
+        mask = orc.select_mask(orc.hamming_scores(q_codes[b][None], cache.read_codes(b).cpu()[None]), init, recent, float(n))
+        ref = orc.masked_attention(q[b:b + 1], ks[b][None], vs[b][None], mask)
+        rel = (out[b] - ref[0]).norm(dim=-1) / ref[0].norm(dim=-1)
+        assert float(rel.max()) < GATHER_REL_L2, (b, rel.tolist())
+
+
 # ------------------------------------------------------------------------------------------
 # the whole step
 # ------------------------------------------------------------------------------------------
