@@ -446,11 +446,11 @@ hash_decode_kernel(const HashDecodeParams p) {
 
 // ------------------------------------------------------------------------------------------
 // Batched variant: a CTA evaluates 16 sequences of its (head, side) at once, each layer a GEMM of 16 rows on the tensor
-// cores (mma.sync m16n8k16; the 128 rows of a tcgen05 tile would be seven eighths padding). Weights stay in registers in
-// the form in which the matrix instruction takes them: a warp owns one or two n-tiles (8 outputs) of a hidden layer, and in
-// the last layer n-tile w % 4 over a part of the inputs. The order of the inputs inside a product is
-// free, so a lane's share of 32 inputs is 8 consecutive ones: one 16-byte load each of weights and activations feeds two
-// k-steps.
+// cores (mma.sync m16n8k16; the 128 rows of a tcgen05 tile would be seven eighths padding). Weights stay in registers (but
+// for 72 bytes a thread that the build for fp32 weights spills) in the form in which the matrix instruction takes them: a warp
+// owns one or two n-tiles (8 outputs) of a hidden layer, and in the last layer n-tile w % 4 over a part of the inputs. The
+// order of the inputs inside a product is free, so a lane's share of 32 inputs is 8 consecutive ones: one 16-byte load each of
+// weights and activations feeds two k-steps.
 // Precision: products of two bf16 are exact. An activation is split into three bf16 (24 bits of mantissa), an fp32 weight
 // too; of their nine products the three smallest are left out, the larger two of them at most 2^-22 of the whole each (cut
 // off parts lie below 2^-7 and 2^-15 of it). The products of the leading parts are summed up by the matrix instruction over

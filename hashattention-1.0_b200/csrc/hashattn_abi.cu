@@ -86,13 +86,14 @@ AttSplit att_split(const ha_shape_t* s, const ha_budget_t* b) {
     return a;
 }
 
-// Small steps (config-1-like: the gather of 41 K rows takes about as long as the hand-over to a merge kernel
-// and the merge together) run the gather as clusters of 8 CTAs x 256 threads per (sequence, head), which merge
-// through distributed shared memory: no partials, no merge kernel.
+// Rounds of 64 rows that each of the 8 CTAs of a cluster takes.
 long long cluster_gather_rounds(long long rows) {
     const long long per_cta = (rows + kAttClusterCtas - 1) / kAttClusterCtas, round = kAttClusterThreads / 16 * kAttRowsPerWorker;  // 64
     return std::max(1ll, (per_cta + round - 1) / round);
 }
+// Small steps (the gather of 41 K rows takes about as long as the hand-over to a merge kernel
+// and the merge together) run the gather as clusters of 8 CTAs x 256 threads per (sequence, head), which merge
+// through distributed shared memory: no partials, no merge kernel.
 AttSplit att_split_launch(const ha_shape_t* s, const ha_budget_t* b) {
     AttSplit a = att_split(s, b);
     long long rows = (long long)s->sel_stride + b->init_budget + b->recent_budget;
@@ -267,7 +268,7 @@ void prefer_carveout(K kernel, int kernel_id, int percent) {
 // Scoring, histograms and the plan (score_hist_kernel) on the kv-heads [p.kvh0, p.kvh0 + nkvh).
 cudaError_t launch_score_hist(const ha_shape_t* shape, int chunk_pages, const SelectParams& p, int nkvh, cudaStream_t s) {
     const dim3 grid(p.nchunks, nkvh, shape->batch);
-    prefer_carveout(score_hist_kernel<1>, 0, 40);   // 4 CTAs x 8 KB
+    prefer_carveout(score_hist_kernel<1>, 0, 40);   // 4 CTAs x 4.2 KB
     prefer_carveout(score_hist_kernel<2>, 1, 100);  // 6 CTAs x 37 KB
     prefer_carveout(score_hist_kernel<4>, 2, 100);
     switch (chunk_pages) {
@@ -807,7 +808,7 @@ int ha_hash_prefill(const ha_shape_t* shape, const ha_hash_weights_t* weights,
         // 64 elements x 128 rows, 128-byte swizzle
         CUtensorMap k_map;
         if (!encode_key_map(&k_map, k_pages, (uint64_t)shape->num_pages * shape->num_kv_heads * kPage)) return HA_ERR_LAUNCH;
-        // one CTA per SM; the kernel cuts the (head, tile) pairs into that many equal ranges
+        // one CTA per SM; the kernel cuts the (head, tile) pairs into that many ranges of equal cost
         const int Hq = shape->num_kv_heads * kGroup;
         const long long tiles = (long long)Hq * shape->batch * shape->max_pages * (kPage / kTcTile);
         int dev = 0, sms = 0;

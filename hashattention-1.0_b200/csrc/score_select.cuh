@@ -33,9 +33,10 @@
 // What bounds it: a CTA spends about 1.5 us on its first words and 1.5 us on publishing its counts, so the stream of the
 // others has to cover that. With the words in flight in shared memory (cp.async) six CTAs fit on an SM, where the
 // registers to hold them allowed four: scoring and plan of 32 sequences of 16384 - 65536 tokens x 8 kv-heads take 47.8 us
-// instead of 54.7 (5 CTAs 50.5, 8 47.2), of 4 x 131072 17.7 instead of 18.6 (8 CTAs, with spills: 21.4), of 32 x 20000
-// 21.3 instead of 24.3; the hash words alone would take 28.2, 10.2 and 12.5. Chunks of one round keep them in
-// registers: there the trip through shared memory costs 0.3 us (3 x 9001 - 15000: 5.5 us, else 5.2) and the grid is small.
+// instead of 54.7 (5 CTAs 50.5), of 4 x 131072 17.7 instead of 18.6, of 32 x 20000 21.3 instead of 24.3; the hash words
+// alone would take 28.2, 10.2 and 12.5. (Registers capped as for 8 CTAs, of which the shared memory holds six all the same:
+// 47.2 and, with spills, 21.4.) Chunks of one round keep them in registers: there the trip through shared memory costs 0.3
+// us (3 x 9001 - 15000: 5.5 us, else 5.2) and the grid is small.
 //
 // Layout of a score plane: inside every block of 128 tokens the byte of token 32 it + lane (the it-th
 // token of a lane in the warp's round) sits at offset 4 lane + it, so that a lane stores its four
@@ -300,6 +301,8 @@ __device__ __forceinline__ void select_plan(const SelectParams& p, int b, int kv
     }
     // hand the head over: one count per CTA of select_attend_kernel that will take this plan (a chunk each). Those CTAs run
     // while other units are still being scored; each takes its count back, so the word is zero again when the step is over.
+    // (The totals and sel_cnt are written behind the announcement: they are read by kernels behind select_attend_kernel only,
+    // whose edge CTAs wait for this grid to end.)
     __syncwarp();
     if (lane == 0 && p.ready != nullptr) {
         __threadfence();  // the warp's stores (ordered before this lane by the barrier) are visible device-wide
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(kSelThreads, ROUNDS == 1 ? 4 : kShMinCtas) sco
     const bool active = s_ok && chunk_start < S;
     const SeqRange r = seq_range(s_ok ? S : 1, p.init_budget, p.recent_budget, p.heavy_budget,
                                  p.budget_lens != nullptr ? p.budget_lens[b] : -1);
-    // two rounds of hash words are kept in flight: while one is scored the next is on its way
+    // with several rounds the words of two are in flight: while one is scored the next is on its way
     RoundWords rw;
     StagedRound st[2];
     int pgs[ROUNDS];  // page ids of this warp's half pages, all requested up front

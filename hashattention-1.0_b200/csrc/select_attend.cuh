@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kSaThreads, kMinCtas) select_attend_kernel(con
         pdl_wait();
     } else if (active) {
         // The scoring kernel in front is still running, but all of its CTAs have started (it lets its dependents go
-        // only then), so the unit's plan arrives without any help from this grid. The wait is bounded all the same.
+        // only then), so the head's plan arrives without any help from this grid. The wait is bounded all the same.
         if (tid == 0) {
             int* word = p.ready + ((size_t)b * p.Hkv + kvh) * kReadyStride + g;
             int v, polls = 0;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kSaThreads, kMinCtas) select_attend_kernel(con
         prefetch_l2(vr + kHeadDim / 2);
     };
     // Tokens above the threshold are certain to be attended: their rows are asked for right here, before the scan
-    // and its barriers (per-unit hand-over only: there the page ids are complete behind the ready word's barrier)
+    // and its barriers (hand-over of the plan only: there the page ids are complete behind the ready word's barrier)
     const bool early = kGather && p.ready != nullptr;
     if constexpr (kGather) {
         if (early) {
