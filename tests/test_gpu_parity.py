@@ -96,6 +96,12 @@ PREFILL_SHAPES = [
     (1, [40000], None),
     (2, [700, 2048, 33], [130, 2047, 0]),
     (8, [3000, 1], None),
+    # as many (head, tile) pairs as a B200 has SMs, 148, and a few more or less, as one sequence and as several: up to there
+    # a CTA takes one at most
+    (1, [37 * 128], None),
+    (1, [37 * 128 + 1], None),
+    (8, [100, 128, 1, 77], None),
+    (8, [100, 128, 1, 77, 129], None),
 ]
 
 
@@ -136,6 +142,35 @@ def test_prefill_shapes_match_the_fp32_hash_mlp(device, hkv, lens, first, bf16_w
                     assert bool((got[h][:f0] == sentinel).all()), (b, h, "tokens in front of first_token were written")
     untouched = cache.hash_pages.to(torch.int64) & 0xFFFFFFFF
     assert bool((untouched[~written] == sentinel).all()), "a slot outside [first_token, S) was written"
+
+
+def test_small_builds_take_one_tile_per_cta(device):
+    """96 (head, tile) pairs, one each for 96 of the SMs, take hardly longer than 32. Cut into ranges of equal cost with the
+    start of a head counted, some CTAs had two and the build took 1.16 times as long (fp32 weights); with one each 1.05."""
+    usa = synthetic.make_usa(32, 128, 3, False)
+
+    def build_us(batch):
+        cache = ha.PagedHashKVCache(batch, 8, 100, device, shuffle_seed=3)
+        synthetic.fill_cache_on_device(cache, [100] * batch, seed=3)
+        ctx = ha.SparseDecodeContext(cache, ha.Budget(16, 0.125, 16), usa.packed(device))
+        ctx.hash_prefill()
+        ctx.check_status()
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+            for _ in range(10):
+                ctx.hash_prefill()
+        times = []
+        for _ in range(20):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end) * 100.0)
+        return min(times[5:])
+
+    three, one = build_us(3), build_us(1)
+    assert three < 1.11 * one, (three, one)
 
 
 PREFILL_RANGES = [
