@@ -636,11 +636,13 @@ def test_two_layer_hash_function_in_the_batched_encoder(device):
 
 
 @pytest.mark.parametrize("batch,bf16_weights,layers", [(5, True, 3), (9, False, 3), (31, True, 2), (32, False, 3), (33, True, 3),
-                                                       (34, False, 2), (6, True, 1), (35, False, 1)])
+                                                       (34, False, 2), (6, True, 1), (35, False, 1), (11, False, 3), (11, True, 1),
+                                                       (11, False, 2)])
 def test_batched_encoder_rows(device, batch, bf16_weights, layers):
-    """The batched encoder at the edges of its tiling: the fewest rows per CTA it is used for (3 with bf16 weights, 5 with
-    fp32 ones), 15 and 16 + 1 (a second pass of one row), a last CTA with fewer rows than the first, every depth of the
-    hash function. Pre-activations, codes and appended rows against the oracle."""
+    """The batched encoder at the edges of its tiling: the fewest rows per CTA it is used for (3 with bf16 weights, 6 with
+    fp32 ones or one layer; with 5 and 3 of these the encoder of single rows), 15 and 16 + 1 (a second pass of one row), a
+    last CTA with fewer rows than the first, every depth of the hash function. Pre-activations, codes and appended rows
+    against the oracle."""
     Hq, Hkv = 32, 8
     lens = [1 + (37 * b) % 300 for b in range(batch)]
     usa = synthetic.make_usa(Hq, 128, 11, bf16_weights, num_layers=layers)
@@ -792,7 +794,7 @@ def test_batched_encoder_on_values_that_are_not_finite(device, bf16_weights, lay
     one = ha.PagedHashKVCache(1, Hkv, 300, device, shuffle_seed=3)
     one.seq_lens.fill_(1)
     single = ha.SparseDecodeContext(one, ha.Budget(16, 0.125, 16), usa.packed(device))
-    many = 8  # the batched encoder is used from 3 (5) sequences per CTA on: the rows are repeated
+    many = 8  # the batched encoder is used from 3 (6) sequences per CTA on: the rows are repeated
     big_cache = ha.PagedHashKVCache(batch * many, Hkv, 300, device, shuffle_seed=3)
     big_cache.seq_lens.fill_(1)
     big_ctx = ha.SparseDecodeContext(big_cache, ha.Budget(16, 0.125, 16), usa.packed(device))
@@ -1147,9 +1149,9 @@ def test_host_buffer_entry_point_equals_device_entry_point(device):
     assert torch.equal(out_dev, out_paged)  # pageable buffers: staged through device copies
 
 
-@pytest.mark.parametrize("batch,bf16_weights", [(5, True), (16, True), (33, True), (9, False)])
+@pytest.mark.parametrize("batch,bf16_weights", [(5, True), (16, True), (33, True), (12, False)])
 def test_host_buffers_of_a_batch_that_takes_the_batched_encoder(device, batch, bf16_weights):
-    """Page-locked rows read over the bus by the batched encoder (3 rows per CTA with bf16 weights, 5 with fp32 ones, and
+    """Page-locked rows read over the bus by the batched encoder (3 rows per CTA with bf16 weights, 6 with fp32 ones, and
     more than one pass): the same bits as from device memory and through staging copies."""
     Hq, Hkv = 32, 8
     lens = [1 + (53 * b) % 200 for b in range(batch)]
