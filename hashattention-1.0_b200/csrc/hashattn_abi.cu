@@ -577,7 +577,7 @@ int ha_workspace_init(const ha_shape_t* shape, const ha_budget_t* budget, void* 
     if (workspace == nullptr) return HA_ERR_WORKSPACE;
     const Workspace w = carve(shape, budget, workspace);
     if (workspace_bytes < w.bytes) return HA_ERR_WORKSPACE;
-    // the arrival counters of the scoring kernel must start at zero (the kernel leaves them at zero);
+    // the arrival counters, totals and ready words of the scoring kernel must start at zero (the kernels leave them at zero);
     // nothing else in the workspace carries state between calls
     if (cudaMemsetAsync(workspace, 0, w.bytes, static_cast<cudaStream_t>(stream)) != cudaSuccess)
         return HA_ERR_LAUNCH;
