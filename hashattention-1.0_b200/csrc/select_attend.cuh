@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kSaThreads, kMinCtas) select_attend_kernel(con
         // The scoring kernel in front is still running, but all of its CTAs have started (it lets its dependents go
         // only then), so the head's plan arrives without any help from this grid. The wait is bounded all the same.
         if (tid == 0) {
-            int* word = p.ready + ((size_t)b * p.Hkv + kvh) * kReadyStride + g;
+            int* word = p.ready + ((size_t)b * p.Hkv + kvh) * kReadyStride + g * kReadyHead;
             int v, polls = 0;
             for (;;) {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
