@@ -295,10 +295,11 @@ __global__ void __launch_bounds__(kThreads, kCluster ? 2 : 6) sparse_gather_kern
         };
         if constexpr (!kPhysical) edges();
         if (first < end) {
-            // five rows per worker where that saves a round over four (79 rows a CTA 13.9 us, with four 14.4; 128 rows 16.2
-            // and 16.0)
+            // five rows per worker where that saves one of two or three rounds of four (79 rows a CTA 13.9 us, with four 14.4;
+            // 128 rows 16.2 and 16.0). More rounds of five take longer than the one they save: 8000 tokens at 1/2, 1, 4 and 8
+            // units, 16.7, 19.0 and 20.6 us, with four 16.5, 18.5 and 19.8
             const int most = (cnt + kAttClusterCtas - 1) / kAttClusterCtas;
-            if ((most + 5 * kWorkers - 1) / (5 * kWorkers) < (most + 4 * kWorkers - 1) / (4 * kWorkers)) heavy(RowsPerWorker<5>());
+            if (most <= 3 * 4 * kWorkers && (most + 5 * kWorkers - 1) / (5 * kWorkers) < (most + 4 * kWorkers - 1) / (4 * kWorkers)) heavy(RowsPerWorker<5>());
             else heavy(RowsPerWorker<4>());
         }
     }

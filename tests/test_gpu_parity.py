@@ -379,6 +379,16 @@ def test_step_through_the_cluster_gather(device, n, init, recent):
         assert float(rel.max()) < GATHER_REL_L2, (b, rel.tolist())
 
 
+@pytest.mark.parametrize("n", [1536, 1544, 2104])
+def test_step_through_many_rounds_of_the_cluster_gather(device, n):
+    """Shares of 192, 193 and 263 list entries per CTA: the last that may go by five rows per worker, and rounds of four. Sets
+    and outputs against the oracle."""
+    lens = [4200, 2500]
+    q, ks, vs = _plain_inputs(61 + n, lens, 8, 2)
+    _, _, ctx, _ = run_step_and_check(device, synthetic.make_usa(8, 128, 3, True), q, ks, vs, ha.Budget(64, float(n), 64))
+    assert ctx.step_path().endswith("sparse_gather (cluster)")
+
+
 # ------------------------------------------------------------------------------------------
 # the whole step
 # ------------------------------------------------------------------------------------------
